@@ -493,12 +493,13 @@ int tomo_net_predict_strided(tomo_net *net, int n, const tomo_net_sample *sample
         NK(tomo::net::features(net->jobs.ptr, cnt, h, net->act[X].ptr, per, net->stream));
         rc = forward(net, v, false);
         if (rc != TOMO_OK) return rc;
-        long long max_nat = 0;
-        for (const auto &j : jobs) max_nat = std::max(max_nat, (long long)j.nz * j.wnx * j.wny);
-        if (stride == 1)
-            NK(tomo::net::tau_to_time(net->jobs.ptr, cnt, h, net->tau.ptr, t_pred + nat, per, net->stream));
-        else
-            NK(tomo::net::tau_to_time_strided(net->jobs.ptr, cnt, h, net->tau.ptr, t_pred + nat, max_nat, net->stream));
+        int max_plane = 1, max_wnx = 1;
+        for (const auto &j : jobs) {
+            max_plane = std::max(max_plane, j.nz * j.wny);
+            max_wnx = std::max(max_wnx, j.wnx);
+        }
+        NK(tomo::net::tau_to_time(net->jobs.ptr, cnt, h, stride, net->tau.ptr, t_pred + nat, max_plane, max_wnx,
+                                  net->stream));
         for (const auto &j : jobs) nat += (long long)j.nz * j.wnx * j.wny;
         i0 += cnt;
     }

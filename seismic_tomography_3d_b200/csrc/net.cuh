@@ -84,11 +84,9 @@ cudaError_t features(const Job *jobs, int njobs, float h, bf16 *x16, long long m
 cudaError_t tau_target(const Job *jobs, int njobs, float h, float *tau, long long max_vox, cudaStream_t st);
 // predicted traveltime tau * s_src * distance into the back-to-back natural layout (0 at
 // distance < h: no ceiling there); jobs with stride > 1 interpolate tau trilinearly between
-// the sampled nodes first (max_nat: the largest window volume)
-cudaError_t tau_to_time(const Job *jobs, int njobs, float h, const float *tau, float *t_out, long long max_vox,
-                        cudaStream_t st);
-cudaError_t tau_to_time_strided(const Job *jobs, int njobs, float h, const float *tau, float *t_out,
-                                long long max_nat, cudaStream_t st);
+// the sampled nodes first (max_plane, max_wnx: the largest nz * wny and wnx of the jobs)
+cudaError_t tau_to_time(const Job *jobs, int njobs, float h, int stride, const float *tau, float *t_out,
+                        int max_plane, int max_wnx, cudaStream_t st);
 
 // Seeded random layered models (training data): one 64^3-like tile per entry of `tiles`,
 // written as slowness into the natural-layout model of size nz x nx x ny.
