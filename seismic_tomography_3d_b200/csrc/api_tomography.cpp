@@ -10,10 +10,6 @@
 #include "internal.hpp"
 #include "ray.cuh"
 
-namespace tomo {
-int rebrick_model(tomo_ctx *ctx);  // api_eikonal.cpp
-}
-
 namespace {
 
 constexpr unsigned long long kSpinLimit = 1ull << 26;
@@ -632,14 +628,14 @@ int update_prepare(tomo_ctx *ctx, const tomo_update_opts *opts)
         CK(ctx->gauss_kernel.ensure(k.size()));
         CK(cudaMemcpyAsync(ctx->gauss_kernel.ptr, k.data(), k.size() * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-        CK(ctx->dm_smooth.ensure(n));
+        if (!tomo::update_fuses(samples)) CK(ctx->dm_smooth.ensure(n));
         CK(cudaStreamSynchronize(ctx->stream));  // k is a host temporary
     }
     return TOMO_OK;
 }
 
-// dm from the CGLS solution, optional smoothing, slowness += dm, re-brick (velocity_out:
-// device array or nullptr).
+// dm from the CGLS solution, optional smoothing, slowness += dm in the natural and the
+// brick-major model (velocity_out: device array or nullptr).
 int update_enqueue_v(tomo_ctx *ctx, const tomo_update_opts *opts, float *velocity_out)
 {
     const int smooth = opts ? opts->smooth : 1;
@@ -650,13 +646,16 @@ int update_enqueue_v(tomo_ctx *ctx, const tomo_update_opts *opts, float *velocit
     CK(tomo::model_dm(ctx->x.ptr, ctx->dm.ptr, g.nx, g.ny, g.nz, g.dx, g.dy, g.dz, ctx->dxt, ctx->dyt, ctx->dzt,
                       ctx->nxt, ctx->nyt, ctx->nzt, m, ctx->stream));
     const float *dm = ctx->dm.ptr;
-    if (smooth) {
+    int fused = smooth ? samples : 1;
+    if (!tomo::update_fuses(fused)) {
         CK(tomo::gaussian_smooth(ctx->dm.ptr, ctx->dm_smooth.ptr, g.nx, g.ny, g.nz, samples, ctx->gauss_kernel.ptr,
                                  ctx->stream));
         dm = ctx->dm_smooth.ptr;
+        fused = 1;
     }
-    CK(tomo::model_apply(ctx->slow.ptr, dm, velocity_out, g.nx, g.ny, g.nz, m, ctx->stream));
-    return tomo::rebrick_model(ctx);
+    CK(tomo::model_update(dm, ctx->slow.ptr, ctx->S.ptr, velocity_out, fused, ctx->gauss_kernel.ptr, g.nx, g.ny, g.nz,
+                          ctx->nxx, ctx->nyy, ctx->nzz, m, ctx->stream));
+    return TOMO_OK;
 }
 
 int update_enqueue(tomo_ctx *ctx, const tomo_update_opts *opts) { return update_enqueue_v(ctx, opts, nullptr); }

@@ -38,10 +38,16 @@ struct UpdateMasks {
 
 cudaError_t model_dm(const float *xdm, float *dm, int nx, int ny, int nz, float dx, float dy, float dz, float dxt,
                      float dyt, float dzt, int nxt, int nyt, int nzt, UpdateMasks m, cudaStream_t st);
+// Whether model_update sums a filter of `samples` by itself; gaussian_smooth does the others.
+bool update_fuses(int samples);
 cudaError_t gaussian_smooth(const float *in, float *out, int nx, int ny, int nz, int samples, const float *kernel,
                             cudaStream_t st);
-cudaError_t model_apply(float *slowness, const float *dm, float *velocity, int nx, int ny, int nz, UpdateMasks m,
-                        cudaStream_t st);
+// Smooths dm with the samples^3 filter `kernel` (samples = 1: dm as it is) and adds it to the
+// slowness inside the masks, natural and brick-major (padded to nxx, nyy, nzz); velocity
+// (may be nullptr) = 1 / slowness.
+cudaError_t model_update(const float *dm, float *slowness, float *bricks, float *velocity, int samples,
+                         const float *kernel, int nx, int ny, int nz, int nxx, int nyy, int nzz, UpdateMasks m,
+                         cudaStream_t st);
 cudaError_t data_residual(const float *dobs, const float *dcal, float *B, int n, int n_total, double *partial,
                           cudaStream_t st);
 

@@ -103,7 +103,21 @@ __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
 
-// trilinear (src/utils/interpolation/trilinear.cpp:3-20), same operation order.
+// trilinear (src/utils/interpolation/trilinear.cpp:3-20), same operation order, from the
+// weights of the upper corners.
+__device__ __forceinline__ float trilinear_weights(float c000, float c001, float c100, float c101, float c010,
+                                                   float c011, float c110, float c111, float xd, float yd, float zd)
+{
+    const float c00 = fadd(fmul(c000, fsub(1.0f, xd)), fmul(c100, xd));
+    const float c01 = fadd(fmul(c001, fsub(1.0f, xd)), fmul(c101, xd));
+    const float c10 = fadd(fmul(c010, fsub(1.0f, xd)), fmul(c110, xd));
+    const float c11 = fadd(fmul(c011, fsub(1.0f, xd)), fmul(c111, xd));
+    const float c0 = fadd(fmul(c00, fsub(1.0f, yd)), fmul(c10, yd));
+    const float c1 = fadd(fmul(c01, fsub(1.0f, yd)), fmul(c11, yd));
+    return fadd(fmul(c0, fsub(1.0f, zd)), fmul(c1, zd));
+}
+
+// The same from the corners' coordinates.
 __device__ __forceinline__ float trilinear_ref(float c000, float c001, float c100, float c101,
                                                float c010, float c011, float c110, float c111,
                                                float x0, float x1, float y0, float y1, float z0,
@@ -112,13 +126,7 @@ __device__ __forceinline__ float trilinear_ref(float c000, float c001, float c10
     const float xd = fdiv(fsub(x, x0), fsub(x1, x0));
     const float yd = fdiv(fsub(y, y0), fsub(y1, y0));
     const float zd = fdiv(fsub(z, z0), fsub(z1, z0));
-    const float c00 = fadd(fmul(c000, fsub(1.0f, xd)), fmul(c100, xd));
-    const float c01 = fadd(fmul(c001, fsub(1.0f, xd)), fmul(c101, xd));
-    const float c10 = fadd(fmul(c010, fsub(1.0f, xd)), fmul(c110, xd));
-    const float c11 = fadd(fmul(c011, fsub(1.0f, xd)), fmul(c111, xd));
-    const float c0 = fadd(fmul(c00, fsub(1.0f, yd)), fmul(c10, yd));
-    const float c1 = fadd(fmul(c01, fsub(1.0f, yd)), fmul(c11, yd));
-    return fadd(fmul(c0, fsub(1.0f, zd)), fmul(c1, zd));
+    return trilinear_weights(c000, c001, c100, c101, c010, c011, c110, c111, xd, yd, zd);
 }
 
 #endif  // __CUDACC__
