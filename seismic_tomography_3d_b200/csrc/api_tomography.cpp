@@ -464,7 +464,7 @@ int tomo_data_residual(tomo_ctx *ctx, double *norm)
         return fail(ctx, TOMO_ERR_INVALID_ARG, "observed data size does not match nshots*nrec of the solve");
     CK(cudaSetDevice(ctx->device));
     const int n = ctx->nshots * ctx->nrec;
-    CK(ctx->norm2.ensure(1));
+    CK(ctx->norm2.ensure(1 + tomo::kNormBlocks));
     CK(tomo::data_residual(ctx->dobs.ptr, ctx->t_recv.ptr, nullptr, n, n, ctx->norm2.ptr, ctx->stream));
     double v = 0.0;
     CK(cudaMemcpyAsync(&v, ctx->norm2.ptr, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -562,7 +562,7 @@ int cgls_prepare(tomo_ctx *ctx, int iterations)
     CK(ctx->cg_r.ensure((size_t)M));
     CK(ctx->cg_p.ensure((size_t)M));
     CK(ctx->hist.ensure((size_t)(iterations > 0 ? iterations : 1)));
-    CK(ctx->norm2.ensure(1));
+    CK(ctx->norm2.ensure(1 + tomo::kNormBlocks));
     int grid = 0;
     CK(tomo::cgls_grid(&grid));
     CK(ctx->partials.ensure((size_t)grid * 3));

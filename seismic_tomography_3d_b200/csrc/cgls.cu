@@ -13,11 +13,11 @@
 // A' has very uneven rows: a model cell is crossed by anything from no ray to thousands
 // (config 3: median 3 non-zeros, maximum 3,206; config 5: 778 on average).  Rows longer
 // than long_row_limit -- 8 x the mean row length, at least kLongRow -- are listed once per
-// call (cgls_long_rows, in row order) and each is summed by a whole block; the 32-lane
-// groups take the rest, so the longest row no longer sets the length of A's.  A fixed
-// limit of kLongRow sent nearly every config-5 row to a block, one row at a time per block:
-// 2.26 ms per iteration there against 1.83 ms with the relative limit and the unrolled
-// gathers (config 3: 0.111 -> 0.094 ms).
+// call (cgls_long_rows, in row order) and summed with eight accumulators a lane; a warp takes
+// one row at a time, long ones first, from its block's share of the rows (spmv_t).  A fixed
+// limit of kLongRow made nearly every config-5 row a long one: 2.26 ms per iteration there
+// against 1.83 ms with the relative limit and the unrolled gathers (config 3: 0.111 ->
+// 0.094 ms).
 #include <cub/cub.cuh>
 #include <thrust/iterator/counting_iterator.h>
 
@@ -67,12 +67,23 @@ __device__ __forceinline__ int long_row_limit(const int *t_ptr, int M)
     return mean8 > kLongRow ? (int)mean8 : kLongRow;
 }
 
-// y = M x for a CSR matrix with `G` lanes per row: FP32 matrix values, FP64 vectors and
-// row sums.  Returns this thread's share of y'y.  kSkipLong: rows longer than long_row
-// are left to spmv_long.  The gathers are unrolled 4 deep (same summation order).
-template <int G, bool kSkipLong = false>
+// One lane's share of a row's product: entries b, b + step, ... of the row, gathers unrolled
+// 4 deep.  x is read through L1: it is rewritten only between grid barriers, whose fence
+// drops the SM's stale lines (30 iterations, 160,000 rays on 5.8 M non-zeros: 2.94 -> 2.70 ms;
+// 160,000 rays of the 401 x 401 x 201 model: 5.71 -> 5.33 ms).
+__device__ __forceinline__ double lane_sum(const int *idx, const float *val, const double *x, int b, int e, int step)
+{
+    double acc = 0.0;
+#pragma unroll 4
+    for (int k = b; k < e; k += step) acc += (double)__ldg(val + k) * x[__ldg(idx + k)];
+    return acc;
+}
+
+// y = A x with `G` lanes per row: FP32 matrix values, FP64 vectors and row sums.  Returns this
+// thread's share of y'y.
+template <int G>
 __device__ __forceinline__ double spmv(const int *ptr, const int *idx, const float *val, const double *x, double *y,
-                                       int nrows, int long_row = 0)
+                                       int nrows)
 {
     const int lane = threadIdx.x & 31;
     const int sub = lane % G;
@@ -82,16 +93,9 @@ __device__ __forceinline__ double spmv(const int *ptr, const int *idx, const flo
     double local = 0.0;
     for (long long it = 0; it < iters; it++) {
         const long long row = gthread / G + it * groups;
+        const bool mine = row < nrows;
         double acc = 0.0;
-        bool mine = row < nrows;
-        if (mine) {
-            const int b = __ldg(ptr + row), e = __ldg(ptr + row + 1);
-            mine = !kSkipLong || e - b <= long_row;
-            if (mine) {
-#pragma unroll 4
-                for (int k = b + sub; k < e; k += G) acc += (double)__ldg(val + k) * __ldcg(x + __ldg(idx + k));
-            }
-        }
+        if (mine) acc = lane_sum(idx, val, x, __ldg(ptr + row) + sub, __ldg(ptr + row + 1), G);
         for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o, G);
         if (mine && sub == 0) {
             y[row] = acc;
@@ -101,40 +105,99 @@ __device__ __forceinline__ double spmv(const int *ptr, const int *idx, const flo
     return local;
 }
 
-// The listed long rows of y = M x, one block per row (block i takes rows i, i + grid, ...
-// of the list).  Returns this thread's share of y'y (thread 0 holds it).
-__device__ __forceinline__ double spmv_long(const int *ptr, const int *idx, const float *val, const double *x,
-                                            double *y, const int *rows, const int *nrows_long, double *sh)
+// r = A' s.  Returns this thread's share of r'r.
+//
+// A block's rows are the listed long rows blockIdx, blockIdx + grid, ... and the rows
+// w + 8 (blockIdx + grid it) of its warps w.  Rows differ a hundredfold in length, so a fixed
+// row per warp left the block waiting for its slowest warp, and a long row summed by the whole
+// block (1-12 elements a thread, two block barriers) took 3.3 us of mostly latency, 5 times in
+// a row.  Here the warps draw rows from a counter in shared memory, long ones first.  A warp
+// sums a long row as the 256 threads of a block would: lane l keeps the eight sums of threads
+// l, l + 32, ... (eight gathers in flight) and adds them in that order.  Every row sum, and
+// with the shares formed afterwards in row order every partial of r'r, is the number that a
+// whole block per long row and a fixed warp per other row give, bit for bit.
+// 30 iterations: 160,000 rays, 5.8 M non-zeros on 62,500 cells 2.70 -> 2.13 ms; 10.7 M on
+// 269,000 cells 5.33 -> 4.89 ms.
+__device__ __forceinline__ double spmv_t(const CglsLaunch &p, const double *x, double *y, double *sh, unsigned *next)
 {
-    double local = 0.0;
-    const int nl = __ldcg(nrows_long);
-    for (int i = blockIdx.x; i < nl; i += gridDim.x) {
-        const int row = __ldcg(rows + i);
-        const int b = __ldg(ptr + row), e = __ldg(ptr + row + 1);
-        double acc = 0.0;
-        for (int k = b + (int)threadIdx.x; k < e; k += blockDim.x)
-            acc += (double)__ldg(val + k) * __ldcg(x + __ldg(idx + k));
-        acc = block_sum(acc, sh);
-        if (threadIdx.x == 0) {
-            y[row] = acc;
-            local += acc * acc;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int limit = long_row_limit(p.t_ptr, p.M);
+    const int nl = __ldcg(p.n_long);
+    const int nlong = nl > (int)blockIdx.x ? (nl - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int step = (int)gridDim.x * kWarps;
+    const int iters = (int)(((long long)p.M + step - 1) / step);
+    const int total = nlong + iters * kWarps;
+    if (threadIdx.x == 0) *next = kWarps;
+    __syncthreads();
+    for (int item = warp; item < total;) {
+        int row = -1, b = 0, e = 0;
+        if (item < nlong) {
+            row = __ldcg(p.long_rows + blockIdx.x + item * gridDim.x);
+            b = __ldg(p.t_ptr + row);
+            e = __ldg(p.t_ptr + row + 1);
+            double a[kWarps];
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) a[w] = 0.0;
+            for (int k = b + lane; k < e; k += kThreads) {
+#pragma unroll
+                for (int w = 0; w < kWarps; w++)
+                    if (k + 32 * w < e) a[w] += (double)__ldg(p.t_val + k + 32 * w) * x[__ldg(p.t_idx + k + 32 * w)];
+            }
+            double t = 0.0;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) {
+                for (int o = 16; o > 0; o >>= 1) a[w] += __shfl_xor_sync(kFull, a[w], o);
+                t += a[w];
+            }
+            if (lane == 0) y[row] = t;
+        } else {
+            const long long r = (long long)((item - nlong) / kWarps) * step + blockIdx.x * kWarps + (item - nlong) % kWarps;
+            if (r < p.M) {
+                row = (int)r;
+                b = __ldg(p.t_ptr + row);
+                e = __ldg(p.t_ptr + row + 1);
+                if (e - b <= limit) {
+                    double acc = lane_sum(p.t_idx, p.t_val, x, b + lane, e, 32);
+                    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+                    if (lane == 0) y[row] = acc;
+                }
+            }
+        }
+        if (lane == 0) item = (int)atomicAdd(next, 1u);
+        item = __shfl_sync(kFull, item, 0);
+    }
+    __syncthreads();
+    // the shares: thread 0 the long rows in list order, lane 0 of a warp its other rows in order
+    double local = 0.0, first = 0.0;
+    if (warp == 0)
+        for (int i0 = 0; i0 < nlong; i0 += 32) {
+            const int i = i0 + lane;
+            const double v = i < nlong ? y[__ldcg(p.long_rows + blockIdx.x + i * gridDim.x)] : 0.0;
+            for (int j = 0; j < min(32, nlong - i0); j++) {
+                const double t = __shfl_sync(kFull, v, j);
+                first += t * t;
+            }
+        }
+    for (int it0 = 0; it0 < iters; it0 += 32) {
+        const long long row = blockIdx.x * kWarps + warp + (long long)(it0 + lane) * step;
+        const bool mine = it0 + lane < iters && row < p.M &&
+                          __ldg(p.t_ptr + row + 1) - __ldg(p.t_ptr + row) <= limit;
+        const double v = mine ? y[row] : 0.0;
+        const unsigned m = __ballot_sync(kFull, mine);
+        for (int j = 0; j < min(32, iters - it0); j++) {
+            const double t = __shfl_sync(kFull, v, j);
+            if ((m >> j) & 1u) local += t * t;
         }
     }
-    return local;
-}
-
-// r = A' s: long rows by blocks, the rest by 32-lane groups.
-__device__ __forceinline__ double spmv_t(const CglsLaunch &p, const double *x, double *y, double *sh)
-{
-    const double l = spmv_long(p.t_ptr, p.t_idx, p.t_val, x, y, p.long_rows, p.n_long, sh);
-    return l + spmv<32, true>(p.t_ptr, p.t_idx, p.t_val, x, y, p.M, long_row_limit(p.t_ptr, p.M));
+    return lane == 0 ? first + local : 0.0;
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kThreads) k_cgls(CglsLaunch p)
+__global__ void __launch_bounds__(kThreads, 4) k_cgls(CglsLaunch p)
 {
     __shared__ double sh[kWarps + 1];
+    __shared__ unsigned next;
     const int nb = gridDim.x;
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long nth = (long long)gridDim.x * blockDim.x;
@@ -145,7 +208,7 @@ __global__ void __launch_bounds__(kThreads) k_cgls(CglsLaunch p)
     for (long long i = tid; i < p.M; i += nth) p.x[i] = 0.0;
     if (!grid_barrier(p.ctrl, p.spin_limit)) return;
     // r = A' s
-    double v = block_sum(spmv_t(p, p.s, p.r, sh), sh);
+    double v = block_sum(spmv_t(p, p.s, p.r, sh, &next), sh);
     if (threadIdx.x == 0) pa[blockIdx.x] = v;
     if (!grid_barrier(p.ctrl, p.spin_limit)) return;
     // p = r, q = A r (= A p)
@@ -176,7 +239,7 @@ __global__ void __launch_bounds__(kThreads) k_cgls(CglsLaunch p)
         // sparse_cgls_gpu's exit test on the r of this iteration (src/utils/cgls/cgls.cu:102)
         if (p.tol > 0.0 && sqrt(rTr) < p.tol) break;
         // r = A' s
-        v = block_sum(spmv_t(p, p.s, p.r, sh), sh);
+        v = block_sum(spmv_t(p, p.s, p.r, sh, &next), sh);
         if (threadIdx.x == 0) pa[blockIdx.x] = v;
         if (!grid_barrier(p.ctrl, p.spin_limit)) return;
         const double rTr_new = grid_sum(pa, nb, sh);

@@ -48,7 +48,10 @@ cudaError_t gaussian_smooth(const float *in, float *out, int nx, int ny, int nz,
 cudaError_t model_update(const float *dm, float *slowness, float *bricks, float *velocity, int samples,
                          const float *kernel, int nx, int ny, int nz, int nxx, int nyy, int nzz, UpdateMasks m,
                          cudaStream_t st);
-cudaError_t data_residual(const float *dobs, const float *dcal, float *B, int n, int n_total, double *partial,
+// B = [dobs - dcal ; 0] (nullptr: not wanted) and norm2[0] = ||dobs - dcal||^2 in FP64; norm2
+// holds 1 + kNormBlocks values.
+constexpr int kNormBlocks = 288;
+cudaError_t data_residual(const float *dobs, const float *dcal, float *B, int n, int n_total, double *norm2,
                           cudaStream_t st);
 
 }  // namespace tomo
