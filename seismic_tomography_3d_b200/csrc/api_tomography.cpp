@@ -254,6 +254,8 @@ RayLaunch ray_launch(tomo_ctx *ctx, const JacGeom &jg)
     const tomo_grid &g = ctx->g;
     RayLaunch rl{};
     rl.T = ctx->T.ptr;
+    for (const auto &d : ctx->shots_h)
+        rl.wide = rl.wide || (long long)d.nbx * d.nby * d.nbz * kBrickNodes >= (1ll << 31);
     rl.shots = ctx->shots_d.ptr;
     rl.nshots = ctx->nshots;
     rl.spos = ctx->spos.ptr;

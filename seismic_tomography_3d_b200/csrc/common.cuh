@@ -27,6 +27,21 @@ enum CtrlSlot : int {
     kCtrlWords = 16,
 };
 
+// Division by a divisor known in advance: with z = RN(1 / y), q = RN(a z), r = a - q y (exact)
+// and RN(q + r z), the IEEE quotient in three operations (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990; Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is known in
+// advance", 2004).  q + r z is within 3 x 2^-25 ulp of a / y, so only quotients that near a
+// midpoint could round the other way; tests/test_divide_cpu.py goes through all of them, for
+// every divisor.  Valid for y in [kDivMin, kDivMax] and a = 0 (the sign of a zero quotient
+// may differ) or 2^-80 <= |a| <= 2^80; other a give a quotient that is not correctly rounded
+// (|a| smaller) or NaN (infinite a).
+constexpr float kDivMin = 0x1p-40f, kDivMax = 0x1p40f;
+
+struct Divisor {
+    float y, z;
+};
+
 #ifdef __CUDACC__
 __device__ __forceinline__ unsigned ld_volatile(const unsigned *p)
 {
@@ -102,6 +117,15 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b); }
+
+// The prepared division above.
+__device__ __forceinline__ Divisor divisor(float y) { return Divisor{y, __frcp_rn(y)}; }
+
+__device__ __forceinline__ float fdiv(float a, const Divisor &d)
+{
+    const float q = __fmul_rn(a, d.z);
+    return __fmaf_rn(__fmaf_rn(-q, d.y, a), d.z, q);
+}
 
 // trilinear (src/utils/interpolation/trilinear.cpp:3-20), same operation order, from the
 // weights of the upper corners.

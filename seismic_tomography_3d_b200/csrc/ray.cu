@@ -17,70 +17,102 @@ namespace tomo {
 
 namespace {
 
-// Traveltime of window-local node (z, x, y) of shot d (brick-major pool).
-__device__ __forceinline__ float t_node(const float *T, const ShotDesc &d, int x, int y, int z)
+template <class D>
+__device__ __forceinline__ int trunc_div(float a, const D &b)
 {
-    const long long b = (z >> 2) + (long long)d.nbz * ((x >> 2) + (long long)d.nbx * (y >> 2));
-    return __ldg(T + d.t_off + b * kBrickNodes + (z & 3) + 4 * (x & 3) + 16 * (y & 3));
+    return (int)fdiv(a, b);
 }
 
-// expand_fdm (least_squares.cpp:11-67) adds a replicated one-node halo: expanded index
-// (i, j, k) reads the cropped node (i-1, j-1, k-1) clamped into the field.  Beyond the
-// halo (undefined in the reference) the clamp continues.
-__device__ __forceinline__ float t_exp(const float *T, const ShotDesc &d, int nz, int i, int j, int k)
-{
-    const int z = min(max(i - 1, 0), nz - 1);
-    const int x = min(max(j - 1, 0), d.wnx - 1);
-    const int y = min(max(k - 1, 0), d.wny - 1);
-    return t_node(T, d, x, y, z);
-}
+// A divisor as the march uses it: prepared (kPrepared), or the plain number.
+template <bool kPrepared>
+struct DivBy {
+    typedef float type;
+    static __device__ __forceinline__ float of(float y) { return y; }
+};
+template <>
+struct DivBy<true> {
+    typedef Divisor type;
+    static __device__ __forceinline__ Divisor of(float y) { return divisor(y); }
+};
 
-__device__ __forceinline__ int trunc_div(float a, float b) { return (int)fdiv(a, b); }
+// One shot's field as the march reads it.  A window-local node's offset in the brick-major
+// field is a sum of one part per axis (t_node's brick index times 64 plus the node in the
+// brick, split by axis): with q = n >> 2 bricks before it, z + 60 q, 4 x + (64 nbz - 16) q and
+// 16 y + (64 nbz nbx - 64) q.  Copied out of the shot's descriptor, whose fields the compiler
+// would load again after every store of a run.  I: the offsets' type -- 32 bits unless a field
+// has 2^31 nodes or more.
+template <class I>
+struct Field {
+    const float *T;
+    int nz, wnx, wny;
+    I sx, sy;
+    __device__ __forceinline__ Field(const float *pool, const ShotDesc &d, int nz_)
+        : T(pool + d.t_off), nz(nz_), wnx(d.wnx), wny(d.wny), sx((I)64 * d.nbz - 16), sy((I)64 * d.nbz * d.nbx - 64)
+    {
+    }
+    __device__ __forceinline__ I zpart(int z) const { return (I)z + (I)60 * (z >> 2); }
+    __device__ __forceinline__ I xpart(int x) const { return (I)4 * x + sx * (x >> 2); }
+    __device__ __forceinline__ I ypart(int y) const { return (I)16 * y + sy * (y >> 2); }
 
-// A window-local node's offset in its shot's brick-major field is a sum of one part per
-// axis (t_node's brick index times 64 plus the node in the brick, split by axis).
-__device__ __forceinline__ int zpart(int z) { return ((z >> 2) << 6) + (z & 3); }
-__device__ __forceinline__ int xpart(const ShotDesc &d, int x) { return (((x >> 2) * d.nbz) << 6) + 4 * (x & 3); }
-__device__ __forceinline__ long long ypart(const ShotDesc &d, int y)
-{
-    return (((long long)(y >> 2) * d.nbz * d.nbx) << 6) + 16 * (y & 3);
-}
+    // expand_fdm (least_squares.cpp:11-67) adds a replicated one-node halo: expanded index
+    // (i, j, k) reads the cropped node (i-1, j-1, k-1) clamped into the field.  Beyond the
+    // halo (undefined in the reference) the clamp continues.
+    __device__ __forceinline__ float at_expanded(int i, int j, int k) const
+    {
+        return __ldg(T + ypart(min(max(k - 1, 0), wny - 1)) + xpart(min(max(j - 1, 0), wnx - 1)) +
+                     zpart(min(max(i - 1, 0), nz - 1)));
+    }
 
-// The six axis neighbours of expanded node (i, j, k), each read as t_exp reads it (clamped
-// per axis), from nine per-axis parts instead of six full index computations.
-__device__ __forceinline__ void t_stencil(const float *T, const ShotDesc &d, int nz, int i, int j, int k, float &zm,
-                                          float &zp, float &xm, float &xp, float &ym, float &yp)
-{
-    const float *Tb = T + d.t_off;
-    const int z0 = i - 1, x0 = j - 1, y0 = k - 1;
-    const int Zc = zpart(min(max(z0, 0), nz - 1)), Zm = zpart(min(max(z0 - 1, 0), nz - 1)),
-              Zp = zpart(min(max(z0 + 1, 0), nz - 1));
-    const int Xc = xpart(d, min(max(x0, 0), d.wnx - 1)), Xm = xpart(d, min(max(x0 - 1, 0), d.wnx - 1)),
-              Xp = xpart(d, min(max(x0 + 1, 0), d.wnx - 1));
-    const long long Yc = ypart(d, min(max(y0, 0), d.wny - 1)), Ym = ypart(d, min(max(y0 - 1, 0), d.wny - 1)),
-                    Yp = ypart(d, min(max(y0 + 1, 0), d.wny - 1));
-    zm = __ldg(Tb + Yc + (Zm + Xc));
-    zp = __ldg(Tb + Yc + (Zp + Xc));
-    xm = __ldg(Tb + Yc + (Zc + Xm));
-    xp = __ldg(Tb + Yc + (Zc + Xp));
-    ym = __ldg(Tb + Ym + (Zc + Xc));
-    yp = __ldg(Tb + Yp + (Zc + Xc));
-}
+    // The six axis neighbours of expanded node (i, j, k), each read as at_expanded reads it
+    // (clamped per axis).
+    __device__ __forceinline__ void stencil(int i, int j, int k, float &zm, float &zp, float &xm, float &xp, float &ym,
+                                            float &yp) const
+    {
+        const int z0 = i - 1, x0 = j - 1, y0 = k - 1;
+        const I Zc = zpart(min(max(z0, 0), nz - 1)), Zm = zpart(min(max(z0 - 1, 0), nz - 1)),
+                Zp = zpart(min(max(z0 + 1, 0), nz - 1));
+        const I Xc = xpart(min(max(x0, 0), wnx - 1)), Xm = xpart(min(max(x0 - 1, 0), wnx - 1)),
+                Xp = xpart(min(max(x0 + 1, 0), wnx - 1));
+        const I Yc = ypart(min(max(y0, 0), wny - 1)), Ym = ypart(min(max(y0 - 1, 0), wny - 1)),
+                Yp = ypart(min(max(y0 + 1, 0), wny - 1));
+        zm = __ldg(T + (Yc + Xc + Zm));
+        zp = __ldg(T + (Yc + Xc + Zp));
+        xm = __ldg(T + (Yc + Zc + Xm));
+        xp = __ldg(T + (Yc + Zc + Xp));
+        ym = __ldg(T + (Xc + Zc + Ym));
+        yp = __ldg(T + (Xc + Zc + Yp));
+    }
+};
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) k_ray_march(RayLaunch p)
+// kPrepared: divisions by prepared divisors (common.cuh) instead of IEEE divisions, the same
+// quotients in 3 instructions of 12.  A step has twelve: nine by the grid and cell spacings,
+// prepared once per thread, and three by the gradient's norm, which share one reciprocal.  The
+// march is bound by issue (316 instructions a step), and its divisions were a third of them:
+// 160,000 rays of the 201 x 201 x 101 model 2.2 -> 1.5 ms, of the 401 x 401 x 201 model 4.4 ->
+// 3.4 ms, the second 3.0 ms with 4 CTAs an SM, whose rays share more of L1 (7 fit; 6: 3.1, 5:
+// 3.1, 8 with spills: 4.2).  Only quotients of time differences under 2^-80 s would not be exact; such a
+// component moves no position by an ulp.  Chosen when all spacings lie in [kDivMin, kDivMax]
+// (metres); outside it a reciprocal or a remainder could leave the FP32 range.
+template <class I, bool kPrepared>
+__global__ void __launch_bounds__(128, 4) k_ray_march(RayLaunch p)
 {
     const long long nrays = (long long)p.nshots * p.nrec;
     const float rayStep = fmul(0.2f, p.dz);  // least_squares.cpp:203
+    typedef DivBy<kPrepared> By;
+    typedef typename By::type Div;
+    const Div by_dz = By::of(p.dz), by_dx = By::of(p.dx), by_dy = By::of(p.dy);
+    const Div by_dzt = By::of(p.dzt), by_dxt = By::of(p.dxt), by_dyt = By::of(p.dyt);
+    const Div by_2dz = By::of(fmul(2.0f, p.dz)), by_2dx = By::of(fmul(2.0f, p.dx)), by_2dy = By::of(fmul(2.0f, p.dy));
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nrays;
          t += (long long)gridDim.x * blockDim.x) {
         // march order (ray_order): shot by shot, longest (largest receiver time) first
         // within a shot; results stay indexed by the ray itself
         const long long ray = p.order ? (long long)p.order[t] : t;
         const int s = (int)(ray / p.nrec), r = (int)(ray % p.nrec);
-        const ShotDesc &d = p.shots[s];
-        const float ox = fmul((float)d.wx0, p.dx), oy = fmul((float)d.wy0, p.dy);
+        const Field<I> F(p.T, p.shots[s], p.nz);
+        const float ox = fmul((float)p.shots[s].wx0, p.dx), oy = fmul((float)p.shots[s].wy0, p.dy);
         const float sxg = p.spos[s], syg = p.spos[p.nshots + s], sz = p.spos[2 * p.nshots + s];
         const float sx = fsub(sxg, ox), sy = fsub(syg, oy);
         // source cell (least_squares.cpp:197-201) and source floor node (stall guard)
@@ -89,16 +121,18 @@ __global__ void __launch_bounds__(128) k_ray_march(RayLaunch p)
 
         float zi = p.rz[r], xi = fsub(p.rx[r], ox), yi = fsub(p.ry[r], oy);
         uint2 *runs = p.runs + ray * (long long)p.cap_runs;
-        int nr = 0, L = 0, st = kRayCapped;
+        int nr = 0, nw = 0, L = 0, st = kRayCapped;  // nr: runs opened, nw: runs written
         bool overflow = false;
+        // Steps in the current cell are counted.  The four cells most recently entered keep
+        // their counts in registers (a ray running along a cell face alternates between two or
+        // three cells, whose steps go to one run each), and a run is written once, when its cell
+        // leaves the four: a store nobody waits for.  (Counting in the run array itself put a
+        // load, an add and a store to global memory on nearly every step of a warp, since some
+        // lane changes cells: 160,000 rays of the 401 x 401 x 201 model 5.2 -> 4.4 ms.)
         unsigned cur = 0xffffffffu, cnt = 0;
-        int ci = -1;  // run that collects the steps in cell `cur`
-        // The four cells most recently entered and their runs: a ray running along a cell
-        // face alternates between two or three cells, and their steps go to one run each
-        // instead of a new run per re-entry (the per-cell totals are the same).
         unsigned c0 = 0xffffffffu, c1 = 0xffffffffu, c2 = 0xffffffffu, c3 = 0xffffffffu;
-        int r0 = -1, r1 = -1, r2 = -1, r3 = -1;
-        if (xi < 0.0f || yi < 0.0f || xi > fmul((float)(d.wnx - 1), p.dx) || yi > fmul((float)(d.wny - 1), p.dy)) {
+        unsigned n0 = 0, n1 = 0, n2 = 0, n3 = 0;
+        if (xi < 0.0f || yi < 0.0f || xi > fmul((float)(F.wnx - 1), p.dx) || yi > fmul((float)(F.wny - 1), p.dy)) {
             st = kRayOutside;  // receiver outside this shot's window
             L = p.max_steps;   // skip the march
         }
@@ -107,33 +141,34 @@ __global__ void __launch_bounds__(128) k_ray_march(RayLaunch p)
         int iz = trunc_div(zi, p.dz), ix = trunc_div(xi, p.dx), iy = trunc_div(yi, p.dy);
         int cap = p.max_steps;
         if (p.smin && L == 0) {
-            const float t0 = t_exp(p.T, d, p.nz, iz + 1, ix + 1, iy + 1);
+            const float t0 = F.at_expanded(iz + 1, ix + 1, iy + 1);
             const float smin = *p.smin;
             if (smin > 0.0f) {
                 const float c = t0 * (p.length_factor / (smin * rayStep)) + 256.0f;
                 if (c < (float)cap) cap = (int)c;
             }
         }
-        const float two_dz = fmul(2.0f, p.dz), two_dx = fmul(2.0f, p.dx), two_dy = fmul(2.0f, p.dy);
         while (L < cap) {
             const int i = iz + 1, j = ix + 1, k = iy + 1;
             float tzm, tzp, txm, txp, tym, typ;
-            t_stencil(p.T, d, p.nz, i, j, k, tzm, tzp, txm, txp, tym, typ);
-            const float dTz = fdiv(fsub(tzp, tzm), two_dz);
-            const float dTx = fdiv(fsub(txp, txm), two_dx);
-            const float dTy = fdiv(fsub(typ, tym), two_dy);
+            F.stencil(i, j, k, tzm, tzp, txm, txp, tym, typ);
+            const float dTz = fdiv(fsub(tzp, tzm), by_2dz);
+            const float dTx = fdiv(fsub(txp, txm), by_2dx);
+            const float dTy = fdiv(fsub(typ, tym), by_2dy);
             const float norm = __fsqrt_rn(fadd(fadd(fmul(dTx, dTx), fmul(dTy, dTy)), fmul(dTz, dTz)));
-            zi = fsub(zi, fdiv(fmul(rayStep, dTz), norm));
-            xi = fsub(xi, fdiv(fmul(rayStep, dTx), norm));
-            yi = fsub(yi, fdiv(fmul(rayStep, dTy), norm));
+            const Div by_norm = By::of(norm);
+            zi = fsub(zi, fdiv(fmul(rayStep, dTz), by_norm));
+            xi = fsub(xi, fdiv(fmul(rayStep, dTx), by_norm));
+            yi = fsub(yi, fdiv(fmul(rayStep, dTy), by_norm));
             if (!isfinite(zi) || !isfinite(xi) || !isfinite(yi)) {
                 st = kRayNonFinite;
                 break;
             }
-            iz = trunc_div(zi, p.dz);
-            ix = trunc_div(xi, p.dx);
-            iy = trunc_div(yi, p.dy);
-            const int im = trunc_div(zi, p.dzt), jm = trunc_div(fadd(xi, ox), p.dxt), km = trunc_div(fadd(yi, oy), p.dyt);
+            iz = trunc_div(zi, by_dz);
+            ix = trunc_div(xi, by_dx);
+            iy = trunc_div(yi, by_dy);
+            const int im = trunc_div(zi, by_dzt), jm = trunc_div(fadd(xi, ox), by_dxt),
+                      km = trunc_div(fadd(yi, oy), by_dyt);
             if (im < 0 || im >= p.nzt || jm < 0 || jm >= p.nxt || km < 0 || km >= p.nyt) {
                 st = kRayOutside;
                 break;
@@ -143,21 +178,23 @@ __global__ void __launch_bounds__(128) k_ray_march(RayLaunch p)
             if (cell == cur) {
                 ++cnt;
             } else {
-                if (cnt && ci >= 0) runs[ci].y += cnt;
-                int hit = cell == c0 ? r0 : cell == c1 ? r1 : cell == c2 ? r2 : cell == c3 ? r3 : -1;
-                if (hit < 0) {
+                // the steps so far to their cell (one of the four, unless it found no room)
+                n0 += cur == c0 ? cnt : 0u;
+                n1 += cur == c1 ? cnt : 0u;
+                n2 += cur == c2 ? cnt : 0u;
+                n3 += cur == c3 ? cnt : 0u;
+                if (cell != c0 && cell != c1 && cell != c2 && cell != c3) {
                     if (nr < p.cap_runs) {
-                        runs[nr] = make_uint2(cell, 0u);
-                        hit = nr++;
-                        c3 = c2; r3 = r2;
-                        c2 = c1; r2 = r1;
-                        c1 = c0; r1 = r0;
-                        c0 = cell; r0 = hit;
+                        if (nr >= 4) runs[nw++] = make_uint2(c3, n3);
+                        nr++;
+                        c3 = c2; n3 = n2;
+                        c2 = c1; n2 = n1;
+                        c1 = c0; n1 = n0;
+                        c0 = cell; n0 = 0;
                     } else {
                         overflow = true;
                     }
                 }
-                ci = hit;
                 cur = cell;
                 cnt = 1;
             }
@@ -174,10 +211,14 @@ __global__ void __launch_bounds__(128) k_ray_march(RayLaunch p)
                 break;
             }
         }
-        if (cnt && ci >= 0) runs[ci].y += cnt;
         if (overflow) {
             st = kRayOverflow;
             nr = 0;
+        } else {
+            if (nr >= 4) runs[nw++] = make_uint2(c3, n3 + (cur == c3 ? cnt : 0u));
+            if (nr >= 3) runs[nw++] = make_uint2(c2, n2 + (cur == c2 ? cnt : 0u));
+            if (nr >= 2) runs[nw++] = make_uint2(c1, n1 + (cur == c1 ? cnt : 0u));
+            if (nr >= 1) runs[nw++] = make_uint2(c0, n0 + (cur == c0 ? cnt : 0u));
         }
         p.nuniq[ray] = nr;  // raw run count; k_ray_sort sorts, merges and rewrites it
         p.status[ray] = st;
@@ -379,7 +420,16 @@ static int grid_for(long long n, int threads)
 
 cudaError_t ray_march(const RayLaunch &p, cudaStream_t st)
 {
-    k_ray_march<<<grid_for((long long)p.nshots * p.nrec, 128), 128, 0, st>>>(p);
+    const int grid = grid_for((long long)p.nshots * p.nrec, 128);
+    bool prepared = true;
+    for (const float y : {p.dx, p.dy, p.dz, p.dxt, p.dyt, p.dzt, 2.0f * p.dx, 2.0f * p.dy, 2.0f * p.dz})
+        prepared = prepared && y >= kDivMin && y <= kDivMax;
+    if (!prepared)
+        k_ray_march<long long, false><<<grid, 128, 0, st>>>(p);
+    else if (p.wide)
+        k_ray_march<long long, true><<<grid, 128, 0, st>>>(p);
+    else
+        k_ray_march<int, true><<<grid, 128, 0, st>>>(p);
     return cudaGetLastError();
 }
 

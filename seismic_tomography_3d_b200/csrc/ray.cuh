@@ -22,6 +22,7 @@ enum RayStatus : int {
 struct RayLaunch {
     const int *order;     // rays in march order (nullptr: natural order)
     const float *T;
+    int wide;             // some field has 2^31 nodes or more (64-bit offsets)
     const ShotDesc *shots;
     int nshots;
     const float *spos;    // 3*nshots: x | y | z (metres)
