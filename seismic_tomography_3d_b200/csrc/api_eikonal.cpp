@@ -138,7 +138,7 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
     std::vector<int> tab;
     std::vector<unsigned> shot_tiles;  // per shot and sweep: the sweep's tile count
     int tab_base[16] = {}, tab_nd[16] = {};
-    long long nflags = 0;
+    long long nflags = 0, widest = 0;
     if (tiled) {
         auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
         for (tomo::FsmShot &f : fs) {
@@ -162,11 +162,14 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
             tab_base[q] = (int)tab.size();
             tab_nd[q] = nd;
             long long run = 0;
-            for (int dg = 0; dg < nd; dg++)
+            for (int dg = 0; dg < nd; dg++) {
+                const long long before = run;
                 for (int s = 0; s < nshots; s++) {
                     tab.push_back((int)run);
                     run += tomo::fsm_diag_count(dg, A[(size_t)s], B[(size_t)s], C[(size_t)s]);
                 }
+                widest = std::max(widest, run - before);
+            }
             if (run >= (1ll << 31)) return fail(ctx, TOMO_ERR_CAPACITY, "too many sweep tiles for one NGB batch");
             tab.push_back((int)run);
         }
@@ -180,10 +183,10 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
     }
     CK(ctx->fsm_T.ensure((size_t)total));
     CK(ctx->fsm_shots.ensure((size_t)nshots));
-    CK(ctx->fsm_bar.ensure((size_t)2 * ngroups + 16 + 16 * (size_t)nshots));
+    CK(ctx->fsm_bar.ensure((size_t)2 * ngroups + 17 + 16 * (size_t)nshots));
     CK(cudaMemcpyAsync(ctx->fsm_shots.ptr, fs.data(), fs.size() * sizeof(tomo::FsmShot), cudaMemcpyHostToDevice,
                        ctx->stream));
-    CK(cudaMemsetAsync(ctx->fsm_bar.ptr, 0, (2 * ngroups + 16 + 16 * (size_t)nshots) * sizeof(unsigned),
+    CK(cudaMemsetAsync(ctx->fsm_bar.ptr, 0, (2 * ngroups + 17 + 16 * (size_t)nshots) * sizeof(unsigned),
                        ctx->stream));
     CK(cudaMemsetAsync(ctx->ctrl.ptr, 0, tomo::kCtrlWords * sizeof(unsigned), ctx->stream));
     CK(cudaMemsetAsync(ctx->stats.ptr, 0, 2 * sizeof(unsigned long long), ctx->stream));
@@ -203,6 +206,10 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
     p.dz2dy2 = p.dz2i * p.dy2i;
     p.dx2dy2 = p.dx2i * p.dy2i;
     p.dsum = p.dz2i + p.dx2i + p.dy2i;
+    p.by_zx = tomo::prepare_divisor(p.dz2i + p.dx2i);
+    p.by_zy = tomo::prepare_divisor(p.dz2i + p.dy2i);
+    p.by_xy = tomo::prepare_divisor(p.dx2i + p.dy2i);
+    p.by_sum = tomo::prepare_divisor(p.dsum);
     p.T = ctx->fsm_T.ptr;
     p.shots = ctx->fsm_shots.ptr;
     p.nshots = nshots;
@@ -219,8 +226,9 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
         p.flags = ctx->fsm_flags.ptr;
         p.cursors = ctx->fsm_bar.ptr + 2;
         p.shot_done = ctx->fsm_bar.ptr + 2 * ngroups + 16;
+        p.nan = p.shot_done + 16 * (size_t)nshots;
         p.shot_tiles = reinterpret_cast<const unsigned *>(ctx->fsm_tab.ptr + tab.size());
-        p.sweep_barrier = nshots == 1 ? 1 : 0;  // 64 shots: 55.4 ms with the counts, 58.3 with barriers
+        p.widest = (int)widest;
     }
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
     int grid = 0;

@@ -42,6 +42,9 @@ struct Divisor {
     float y, z;
 };
 
+// On the host (IEEE division rounds to nearest).
+inline Divisor prepare_divisor(float y) { return Divisor{y, 1.0f / y}; }
+
 #ifdef __CUDACC__
 __device__ __forceinline__ unsigned ld_volatile(const unsigned *p)
 {
@@ -125,6 +128,19 @@ __device__ __forceinline__ float fdiv(float a, const Divisor &d)
 {
     const float q = __fmul_rn(a, d.z);
     return __fmaf_rn(__fmaf_rn(-q, d.y, a), d.z, q);
+}
+
+// Square root: the hardware's reciprocal root r gives g = a r and h = r / 2, and one step with
+// the exact residual a - g g corrects g (Markstein 1990): five operations, the IEEE root for
+// every a in [2^-102, 2^126) (tests/test_sqrt_gpu.py goes through all of them) and NaN below
+// zero.  Below 2^-102 it can be an ulp off, and a = 0 is set apart.
+__device__ __forceinline__ float fsqrt(float a)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    const float g = __fmul_rn(a, r), h = __fmul_rn(0.5f, r);
+    const float s = __fmaf_rn(__fmaf_rn(-g, g, a), h, g);
+    return a == 0.0f ? a : s;
 }
 
 // trilinear (src/utils/interpolation/trilinear.cpp:3-20), same operation order, from the

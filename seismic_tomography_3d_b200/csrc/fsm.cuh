@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "common.cuh"
 #include "fim.cuh"
 
 namespace tomo {
@@ -74,6 +75,8 @@ struct FsmLaunch {
     int nx, ny, nz;
     float dx, dy, dz;
     float dz2i, dx2i, dy2i, dz2dx2, dz2dy2, dx2dy2, dsum;  // host-computed as the reference
+    // divisors of the candidates, prepared: dz2i + dx2i, dz2i + dy2i, dx2i + dy2i and dsum
+    Divisor by_zx, by_zy, by_xy, by_sum;
     float *T;                 // sweep pool: per shot (nz+2)(wnx+2)(wny+2), z fastest
     const FsmShot *shots;
     int nshots;
@@ -92,9 +95,12 @@ struct FsmLaunch {
     int tab_base[16], tab_nd[16];
     unsigned *flags;          // per tile: last sweep (q + 1) that finished it
     unsigned *cursors;        // 16 tile cursors, zeroed before the launch
+    unsigned *nan;            // set if a slowness or a seeded time is NaN (zeroed before the launch)
     unsigned *shot_done;      // per shot and sweep: tiles finished (16 x nshots, zeroed)
     const unsigned *shot_tiles;  // per shot and sweep: tiles of the sweep (16 x nshots)
+    int widest;               // most tiles of all shots on one diagonal of a full sweep
     int sweep_barrier;        // 1: a grid barrier between sweeps instead of the per-shot counts
+                              // (set by fsm_solve_tiled)
 };
 
 cudaError_t fsm_solve(const FsmLaunch &p, int *grid_out, cudaStream_t st);
