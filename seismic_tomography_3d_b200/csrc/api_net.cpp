@@ -28,7 +28,7 @@ namespace {
 struct ConvSpec {
     int cin, cout;
     long long w_off, b_off;    // FP32 parameter offsets
-    long long wb_off;          // BF16 weight offsets (forward and flipped share the layout size)
+    long long wb_off, wf_off;  // offsets of the packed BF16 weights (forward, flipped)
 };
 
 // conv order: e1a e1b e2a e2b e3a e3b ba bb d3a d3b d2a d2b d1a d1b
@@ -49,7 +49,7 @@ struct tomo_net {
     bool own_stream = false;
     std::string err;
     ConvSpec conv[kConvs];
-    long long n_params = 0, n_wb = 0, head_off = 0;
+    long long n_params = 0, head_off = 0;
     Buf<float> p, g, m, v;         // FP32 parameters, gradients, Adam moments
     Buf<bf16> wb, wf;              // BF16 forward / flipped (dgrad) weights
     int step = 0;
@@ -160,7 +160,7 @@ int conv_backward(tomo_net *net, int i, int in, int out, int gin, Vol v0)
     NK(tomo::net::conv_wgrad(net->act[in].ptr, dy, net->g.ptr + c.w_off, v, c.cin, c.cout, st));
     NK(tomo::net::bias_grad(dy, net->g.ptr + c.b_off, v.voxels(), c.cout, st));
     if (gin >= 0)
-        NK(tomo::net::conv_fwd(dy, net->wf.ptr + c.wb_off, nullptr, net->grad[gin].ptr, v, c.cout, c.cin, 0, st));
+        NK(tomo::net::conv_fwd(dy, net->wf.ptr + c.wf_off, nullptr, net->grad[gin].ptr, v, c.cout, c.cin, 0, st));
     return TOMO_OK;
 }
 
@@ -203,8 +203,8 @@ int refresh_weights(tomo_net *net)
 {
     for (int i = 0; i < kConvs; i++) {
         const ConvSpec &c = net->conv[i];
-        NK(tomo::net::to_bf16(net->p.ptr + c.w_off, net->wb.ptr + c.wb_off, 27LL * c.cin * c.cout, net->stream));
-        NK(tomo::net::flip_weights(net->p.ptr + c.w_off, net->wf.ptr + c.wb_off, c.cin, c.cout, net->stream));
+        NK(tomo::net::pack_weights(net->p.ptr + c.w_off, net->wb.ptr + c.wb_off, c.cin, c.cout, false, net->stream));
+        NK(tomo::net::pack_weights(net->p.ptr + c.w_off, net->wf.ptr + c.wf_off, c.cin, c.cout, true, net->stream));
     }
     return TOMO_OK;
 }
@@ -322,7 +322,7 @@ int tomo_net_create(int device, void *stream, unsigned long long seed, tomo_net 
     }
     for (int i = 0; i < 2 && e == cudaSuccess; i++) e = cudaEventCreate(&net->ev[i]);
     // parameter layout: per conv [w (cout x 27 x cin), b (cout)], then head [wh (16), bh (1)]
-    long long off = 0, wb = 0;
+    long long off = 0, wb = 0, wf = 0;
     for (int i = 0; i < kConvs; i++) {
         ConvSpec &c = net->conv[i];
         c.cin = kSpec[i][0];
@@ -332,18 +332,19 @@ int tomo_net_create(int device, void *stream, unsigned long long seed, tomo_net 
         c.b_off = off;
         off += c.cout;
         c.wb_off = wb;
-        wb += 27LL * c.cin * c.cout;
+        c.wf_off = wf;
+        wb += tomo::net::packed_weights(c.cin, c.cout);
+        wf += tomo::net::packed_weights(c.cout, c.cin);
     }
     net->head_off = off;
     off += 17;
     net->n_params = off;
-    net->n_wb = wb;
     if (e == cudaSuccess) e = net->p.ensure((size_t)off);
     if (e == cudaSuccess) e = net->g.ensure((size_t)off);
     if (e == cudaSuccess) e = net->m.ensure((size_t)off);
     if (e == cudaSuccess) e = net->v.ensure((size_t)off);
     if (e == cudaSuccess) e = net->wb.ensure((size_t)wb);
-    if (e == cudaSuccess) e = net->wf.ensure((size_t)wb);
+    if (e == cudaSuccess) e = net->wf.ensure((size_t)wf);
     if (e == cudaSuccess) e = net->acc.ensure(2);
     if (e != cudaSuccess) {
         tomo_net_destroy(net);

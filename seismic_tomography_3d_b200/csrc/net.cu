@@ -183,23 +183,6 @@ __global__ void k_bias_grad(const bf16 *dy, float *db, long long n, int c)
     for (int i = threadIdx.x; i < c; i += blockDim.x) atomicAdd(db + i, part[i]);
 }
 
-__global__ void k_flip_weights(const float *w, bf16 *wt, int cin, int cout)
-{
-    const long long n = (long long)cin * 27 * cout;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const int co = (int)(e % cout);
-        const int tap = (int)((e / cout) % 27);
-        const int ci = (int)(e / ((long long)cout * 27));
-        wt[e] = __float2bfloat16_rn(w[((long long)co * 27 + (26 - tap)) * cin + ci]);
-    }
-}
-
-__global__ void k_to_bf16(const float *a, bf16 *b, long long n)
-{
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-        b[e] = __float2bfloat16_rn(a[e]);
-}
-
 __global__ void k_relu_bwd(const bf16 *y, bf16 *dy, long long n)
 {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
@@ -597,18 +580,6 @@ cudaError_t bias_grad(const bf16 *dy, float *db, long long voxels, int c, cudaSt
 {
     if (c > 128) return cudaErrorInvalidValue;
     k_bias_grad<<<grid1(voxels * c / 64, 256), 256, 0, st>>>(dy, db, voxels * c, c);
-    return cudaGetLastError();
-}
-
-cudaError_t flip_weights(const float *w, bf16 *wt, int cin, int cout, cudaStream_t st)
-{
-    k_flip_weights<<<grid1((long long)cin * 27 * cout, 256), 256, 0, st>>>(w, wt, cin, cout);
-    return cudaGetLastError();
-}
-
-cudaError_t to_bf16(const float *a, bf16 *b, long long n, cudaStream_t st)
-{
-    k_to_bf16<<<grid1(n, 256), 256, 0, st>>>(a, b, n);
     return cudaGetLastError();
 }
 

@@ -23,7 +23,7 @@ struct Vol {
     __host__ __device__ long long voxels() const { return (long long)B * D * H * W; }
 };
 
-// y = act(conv3x3x3(x, w) + bias); relu: 0/1; bias may be nullptr.
+// y = act(conv3x3x3(x, w) + bias); w packed (pack_weights); relu: 0/1; bias may be nullptr.
 cudaError_t conv_fwd(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout, int relu,
                      cudaStream_t st);
 // The same convolution on the tcgen05 tensor cores (net_tc.cu): M = 128 voxels per CTA,
@@ -37,9 +37,11 @@ cudaError_t conv_tc_error(unsigned *err, bool reset, cudaStream_t st);
 cudaError_t conv_wgrad(const bf16 *x, const bf16 *dy, float *dw, Vol v, int cin, int cout, cudaStream_t st);
 // db[co] += sum_v dy[v][co]
 cudaError_t bias_grad(const bf16 *dy, float *db, long long voxels, int c, cudaStream_t st);
-// wt[ci][26 - tap][co] = w[co][tap][ci]: the weights of dgrad run as a forward conv
-cudaError_t flip_weights(const float *w, bf16 *wt, int cin, int cout, cudaStream_t st);
-cudaError_t to_bf16(const float *a, bf16 *b, long long n, cudaStream_t st);
+// Weights as conv_fwd reads them: BF16, in the order they lie in shared memory (net_tc.cu).
+// packed_weights: their count for a convolution of cin to cout channels.  flip: the weights of
+// its input gradient (dgrad), run as a forward convolution of cout to cin channels.
+long long packed_weights(int cin, int cout);
+cudaError_t pack_weights(const float *w, bf16 *out, int cin, int cout, bool flip, cudaStream_t st);
 
 // elementwise and resampling (channels-last, c channels)
 cudaError_t relu_bwd(const bf16 *y, bf16 *dy, long long n, cudaStream_t st);      // dy *= (y > 0)
