@@ -39,6 +39,12 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// 16-byte asynchronous global -> shared copy; zeros where !in.
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src, bool in)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+
 struct TileCoord {
     int b, d0, h0, w0;
 };
@@ -70,12 +76,9 @@ __device__ __forceinline__ void stage_halo(const bf16 *x, const Vol &v, int cin,
         const int hv = i >> 1, half = i & 1;
         const int hw = hv % HW, hh = (hv / HW) % HH, hd = hv / (HW * HH);
         const int d = tc.d0 + hd - 1, h = tc.h0 + hh - 1, w = tc.w0 + hw - 1;
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (d >= 0 && d < v.D && h >= 0 && h < v.H && w >= 0 && w < v.W) {
-            const long long vox = (((long long)tc.b * v.D + d) * v.H + h) * v.W + w;
-            val = __ldg(reinterpret_cast<const uint4 *>(x + vox * cin + ci0) + half);
-        }
-        dst[i] = val;
+        const bool in = d >= 0 && d < v.D && h >= 0 && h < v.H && w >= 0 && w < v.W;
+        const long long vox = in ? (((long long)tc.b * v.D + d) * v.H + h) * v.W + w : 0;
+        cp_async16(smem_u32(dst + i), x + vox * cin + ci0 + 8 * half, in);
     }
 }
 
@@ -86,9 +89,13 @@ __device__ __forceinline__ int halo_index(int m, int dd, int dh, int dw)
 }
 
 // wgrad: 9 warps, warp w owns taps 3w .. 3w+2; CTA owns 16 input channels (blockIdx.y) and
-// NM output channels (blockIdx.z), and loops over voxel tiles (blockIdx.x strided).
+// NM output channels (blockIdx.z), and loops over voxel tiles (blockIdx.x strided).  A tile's
+// operand loads (shared-memory bandwidth) would take a quarter of the kernel's time; the rest is
+// waiting for its staging, so what counts is CTAs per SM and copies in flight: registers held to
+// 4 CTAs an SM at NM = 16 and 3 at 32, staging by cp.async.  A gradient of 8 x 64^3 voxels:
+// 6.15 -> 5.30 ms (2 CTAs an SM throughout: 5.37; 5 and 4, with spills: 6.87).
 template <int NM>
-__global__ void __launch_bounds__(288) k_conv_wgrad(const bf16 *x, const bf16 *dy, float *dw, Vol v, int cin,
+__global__ void __launch_bounds__(288, NM == 16 ? 4 : NM == 32 ? 3 : 2) k_conv_wgrad(const bf16 *x, const bf16 *dy, float *dw, Vol v, int cin,
                                                     int cout)
 {
     constexpr int MT = NM / 16;
@@ -117,13 +124,11 @@ __global__ void __launch_bounds__(288) k_conv_wgrad(const bf16 *x, const bf16 *d
             const int r = i / (NM / 8), part = i % (NM / 8);
             const int ww = r % TW, wh = (r / TW) % TH, wd = r / (TW * TH);
             const int d = tc.d0 + wd, h = tc.h0 + wh, ws = tc.w0 + ww;
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (d < v.D && h < v.H && ws < v.W && co0 + part * 8 < cout) {
-                const long long vox = (((long long)tc.b * v.D + d) * v.H + h) * v.W + ws;
-                val = __ldg(reinterpret_cast<const uint4 *>(dy + vox * cout + co0 + part * 8));
-            }
-            *reinterpret_cast<uint4 *>(s_dy + r * DYS + part * 8) = val;
+            const bool in = d < v.D && h < v.H && ws < v.W && co0 + part * 8 < cout;
+            const long long vox = in ? (((long long)tc.b * v.D + d) * v.H + h) * v.W + ws : 0;
+            cp_async16(smem_u32(s_dy + r * DYS + part * 8), dy + (in ? vox * cout + co0 + part * 8 : 0), in);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
 #pragma unroll 1
         for (int kk = 0; kk < kTileVox / 16; kk++) {
@@ -548,7 +553,9 @@ cudaError_t launch_wgrad(const bf16 *x, const bf16 *dy, float *dw, Vol v, int ci
     if (e != cudaSuccess) return e;
     const long long nt = tiles_of(v);
     const int ny = cin / 16, nz = (cout + NM - 1) / NM;
-    long long gx = (2LL * 148 + ny * nz - 1) / (ny * nz);
+    // several times the resident CTAs (2-4 an SM), so that the last ones to finish are short
+    // (4 / 8 / 12 per SM: 5.37 / 5.30 / 5.28 ms per gradient of 8 x 64^3 voxels)
+    long long gx = (8 * 148LL + ny * nz - 1) / (ny * nz);
     if (gx > nt) gx = nt;
     if (gx < 1) gx = 1;
     k_conv_wgrad<NM><<<dim3((unsigned)gx, (unsigned)ny, (unsigned)nz), 288, smem, st>>>(x, dy, dw, v, cin, cout);
