@@ -55,9 +55,9 @@ struct tomo_net {
     int step = 0;
     // activations (BF16) and their gradients, sized for `cap_vox` full-resolution voxels
     long long cap_vox = 0;
-    // forward: x, e1a, e1, p1, e2a, e2, p2, e3a, e3, p3, ba, b, u3, c3, d3a, d3, u2, c2, d2a, d2, u1, c1, d1a, d1
-    Buf<bf16> act[24];
-    Buf<bf16> grad[24];
+    // forward: x, e1a, e1, p1, e2a, e2, p2, e3a, e3, p3, ba, b, c3, d3a, d3, c2, d2a, d2, c1, d1a, d1
+    Buf<bf16> act[21];
+    Buf<bf16> grad[21];
     Buf<float> tau, target;
     Buf<double> acc;
     Buf<tomo::net::Job> jobs;
@@ -82,12 +82,11 @@ int fail(tomo_net *n, int code, const std::string &msg)
 
 // activation slots
 enum Slot {
-    X, E1A, E1, P1, E2A, E2, P2, E3A, E3, P3, BA, BB, U3, C3, D3A, D3, U2, C2, D2A, D2, U1, C1, D1A, D1, NSLOT
+    X, E1A, E1, P1, E2A, E2, P2, E3A, E3, P3, BA, BB, C3, D3A, D3, C2, D2A, D2, C1, D1A, D1, NSLOT
 };
 // channels and level of each slot
-constexpr int kSlotC[NSLOT] = {16, 16, 16, 16, 32, 32, 32, 48, 48, 48, 64, 64,
-                               64, 112, 48, 48, 48, 80, 32, 32, 32, 48, 16, 16};
-constexpr int kSlotL[NSLOT] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 3, 2, 2, 2, 2, 1, 1, 1, 1, 0, 0, 0, 0};
+constexpr int kSlotC[NSLOT] = {16, 16, 16, 16, 32, 32, 32, 48, 48, 48, 64, 64, 112, 48, 48, 80, 32, 32, 48, 16, 16};
+constexpr int kSlotL[NSLOT] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 3, 2, 2, 2, 1, 1, 1, 0, 0, 0};
 
 int ensure_acts(tomo_net *net, long long vox)
 {
@@ -113,8 +112,8 @@ int conv_forward(tomo_net *net, int i, int in, int out, Vol v0)
 {
     const ConvSpec &c = net->conv[i];
     const Vol v = level(v0, kLevel[i]);
-    NK(tomo::net::conv_fwd(net->act[in].ptr, net->wb.ptr + c.wb_off, net->p.ptr + c.b_off, net->act[out].ptr, v, c.cin,
-                           c.cout, 1, net->stream));
+    NK(tomo::net::conv_fwd(net->act[in].ptr, net->wb.ptr + c.wb_off, net->p.ptr + c.b_off, nullptr, net->act[out].ptr, v,
+                           c.cin, c.cout, 1, net->stream));
     return TOMO_OK;
 }
 
@@ -132,35 +131,33 @@ int forward(tomo_net *net, Vol v, bool with_target)
     FWD(4, P2, E3A) FWD(5, E3A, E3)
     NK(tomo::net::pool_fwd(net->act[E3].ptr, net->act[P3].ptr, level(v, 2), 48, st));
     FWD(6, P3, BA) FWD(7, BA, BB)
-    NK(tomo::net::up_fwd(net->act[BB].ptr, net->act[U3].ptr, level(v, 2), 64, st));
-    NK(tomo::net::concat_fwd(net->act[U3].ptr, 64, net->act[E3].ptr, 48, net->act[C3].ptr, level(v, 2).voxels(), st));
+    NK(tomo::net::up_concat(net->act[BB].ptr, 64, net->act[E3].ptr, 48, net->act[C3].ptr, level(v, 2), st));
     FWD(8, C3, D3A) FWD(9, D3A, D3)
-    NK(tomo::net::up_fwd(net->act[D3].ptr, net->act[U2].ptr, level(v, 1), 48, st));
-    NK(tomo::net::concat_fwd(net->act[U2].ptr, 48, net->act[E2].ptr, 32, net->act[C2].ptr, level(v, 1).voxels(), st));
+    NK(tomo::net::up_concat(net->act[D3].ptr, 48, net->act[E2].ptr, 32, net->act[C2].ptr, level(v, 1), st));
     FWD(10, C2, D2A) FWD(11, D2A, D2)
-    NK(tomo::net::up_fwd(net->act[D2].ptr, net->act[U1].ptr, level(v, 0), 32, st));
-    NK(tomo::net::concat_fwd(net->act[U1].ptr, 32, net->act[E1].ptr, 16, net->act[C1].ptr, level(v, 0).voxels(), st));
+    NK(tomo::net::up_concat(net->act[D2].ptr, 32, net->act[E1].ptr, 16, net->act[C1].ptr, level(v, 0), st));
     FWD(12, C1, D1A) FWD(13, D1A, D1)
 #undef FWD
     if (with_target) NK(cudaMemsetAsync(net->acc.ptr, 0, 2 * sizeof(double), st));
     NK(tomo::net::head_fwd(net->act[D1].ptr, net->p.ptr + net->head_off, net->p.ptr + net->head_off + 16, net->tau.ptr,
-                           with_target ? net->target.ptr : nullptr, v.voxels(), 16, net->acc.ptr, st));
+                           with_target ? net->target.ptr : nullptr, v.voxels(), net->acc.ptr, st));
     return TOMO_OK;
 }
 
-// conv layer i backward: dy (grad slot of its output) -> weight/bias gradients and, if
-// gin >= 0, the gradient of its input into grad slot gin
-int conv_backward(tomo_net *net, int i, int in, int out, int gin, Vol v0)
+// conv layer i backward: dz (grad slot of its output, already through its ReLU) -> weight and
+// bias gradients and, if gin >= 0, the gradient of its input into grad slot gin; masked: that
+// input is itself the output of a ReLU, and its gradient is wanted through it
+int conv_backward(tomo_net *net, int i, int in, int out, int gin, bool masked, Vol v0)
 {
     const ConvSpec &c = net->conv[i];
     const Vol v = level(v0, kLevel[i]);
     const cudaStream_t st = net->stream;
-    bf16 *dy = net->grad[out].ptr;
-    NK(tomo::net::relu_bwd(net->act[out].ptr, dy, v.voxels() * c.cout, st));
-    NK(tomo::net::conv_wgrad(net->act[in].ptr, dy, net->g.ptr + c.w_off, v, c.cin, c.cout, st));
-    NK(tomo::net::bias_grad(dy, net->g.ptr + c.b_off, v.voxels(), c.cout, st));
+    const bf16 *dz = net->grad[out].ptr;
+    NK(tomo::net::conv_wgrad(net->act[in].ptr, dz, net->g.ptr + c.w_off, v, c.cin, c.cout, st));
+    NK(tomo::net::bias_grad(dz, net->g.ptr + c.b_off, v.voxels(), c.cout, st));
     if (gin >= 0)
-        NK(tomo::net::conv_fwd(dy, net->wf.ptr + c.wf_off, nullptr, net->grad[gin].ptr, v, c.cout, c.cin, 0, st));
+        NK(tomo::net::conv_fwd(dz, net->wf.ptr + c.wf_off, nullptr, masked ? net->act[in].ptr : nullptr,
+                               net->grad[gin].ptr, v, c.cout, c.cin, 0, st));
     return TOMO_OK;
 }
 
@@ -170,31 +167,27 @@ int backward(tomo_net *net, Vol v)
     int rc;
     NK(cudaMemsetAsync(net->g.ptr, 0, (size_t)net->n_params * sizeof(float), st));
     NK(tomo::net::head_bwd(net->act[D1].ptr, net->p.ptr + net->head_off, net->tau.ptr, net->target.ptr, net->acc.ptr,
-                           net->grad[D1].ptr, net->g.ptr + net->head_off, net->g.ptr + net->head_off + 16, v.voxels(), 16,
-                           st));
-#define BWD(i, a, b, gin)                                        \
-    if ((rc = conv_backward(net, i, a, b, gin, v)) != TOMO_OK) \
+                           net->grad[D1].ptr, net->g.ptr + net->head_off, net->g.ptr + net->head_off + 16, v.voxels(), st));
+#define BWD(i, a, b, gin, masked)                                        \
+    if ((rc = conv_backward(net, i, a, b, gin, masked, v)) != TOMO_OK) \
         return rc;
-    BWD(13, D1A, D1, D1A) BWD(12, C1, D1A, C1)
-    NK(tomo::net::concat_bwd(net->grad[C1].ptr, net->grad[U1].ptr, 32, net->grad[E1].ptr, 16, level(v, 0).voxels(), st));
-    NK(tomo::net::up_bwd(net->grad[U1].ptr, net->grad[D2].ptr, level(v, 0), 32, st));
-    BWD(11, D2A, D2, D2A) BWD(10, C2, D2A, C2)
-    NK(tomo::net::concat_bwd(net->grad[C2].ptr, net->grad[U2].ptr, 48, net->grad[E2].ptr, 32, level(v, 1).voxels(), st));
-    NK(tomo::net::up_bwd(net->grad[U2].ptr, net->grad[D3].ptr, level(v, 1), 48, st));
-    BWD(9, D3A, D3, D3A) BWD(8, C3, D3A, C3)
-    NK(tomo::net::concat_bwd(net->grad[C3].ptr, net->grad[U3].ptr, 64, net->grad[E3].ptr, 48, level(v, 2).voxels(), st));
-    NK(tomo::net::up_bwd(net->grad[U3].ptr, net->grad[BB].ptr, level(v, 2), 64, st));
-    BWD(7, BA, BB, BA) BWD(6, P3, BA, P3)
-    // E3's gradient: skip path (already in grad[E3]) + pooling path
-    NK(tomo::net::pool_bwd(net->grad[P3].ptr, net->grad[E3A].ptr, level(v, 2), 48, st));
-    NK(tomo::net::add_into(net->grad[E3].ptr, net->grad[E3A].ptr, level(v, 2).voxels() * 48, st));
-    BWD(5, E3A, E3, E3A) BWD(4, P2, E3A, P2)
-    NK(tomo::net::pool_bwd(net->grad[P2].ptr, net->grad[E2A].ptr, level(v, 1), 32, st));
-    NK(tomo::net::add_into(net->grad[E2].ptr, net->grad[E2A].ptr, level(v, 1).voxels() * 32, st));
-    BWD(3, E2A, E2, E2A) BWD(2, P1, E2A, P1)
-    NK(tomo::net::pool_bwd(net->grad[P1].ptr, net->grad[E1A].ptr, level(v, 0), 16, st));
-    NK(tomo::net::add_into(net->grad[E1].ptr, net->grad[E1A].ptr, level(v, 0).voxels() * 16, st));
-    BWD(1, E1A, E1, E1A) BWD(0, X, E1A, -1)
+    BWD(13, D1A, D1, D1A, true) BWD(12, C1, D1A, C1, false)
+    NK(tomo::net::up_bwd(net->grad[C1].ptr, 48, net->act[D2].ptr, net->grad[D2].ptr, 32, level(v, 0), st));
+    BWD(11, D2A, D2, D2A, true) BWD(10, C2, D2A, C2, false)
+    NK(tomo::net::up_bwd(net->grad[C2].ptr, 80, net->act[D3].ptr, net->grad[D3].ptr, 48, level(v, 1), st));
+    BWD(9, D3A, D3, D3A, true) BWD(8, C3, D3A, C3, false)
+    NK(tomo::net::up_bwd(net->grad[C3].ptr, 112, net->act[BB].ptr, net->grad[BB].ptr, 64, level(v, 2), st));
+    BWD(7, BA, BB, BA, true) BWD(6, P3, BA, P3, false)
+    // the encoder outputs' gradients: skip path (in the concatenation's) + pooling path
+    NK(tomo::net::skip_bwd(net->grad[C3].ptr, 112, net->grad[P3].ptr, net->act[E3].ptr, net->grad[E3].ptr, 48, level(v, 2),
+                           st));
+    BWD(5, E3A, E3, E3A, true) BWD(4, P2, E3A, P2, false)
+    NK(tomo::net::skip_bwd(net->grad[C2].ptr, 80, net->grad[P2].ptr, net->act[E2].ptr, net->grad[E2].ptr, 32, level(v, 1),
+                           st));
+    BWD(3, E2A, E2, E2A, true) BWD(2, P1, E2A, P1, false)
+    NK(tomo::net::skip_bwd(net->grad[C1].ptr, 48, net->grad[P1].ptr, net->act[E1].ptr, net->grad[E1].ptr, 16, level(v, 0),
+                           st));
+    BWD(1, E1A, E1, E1A, true) BWD(0, X, E1A, -1, false)
 #undef BWD
     return TOMO_OK;
 }

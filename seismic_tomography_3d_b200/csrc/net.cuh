@@ -23,13 +23,11 @@ struct Vol {
     __host__ __device__ long long voxels() const { return (long long)B * D * H * W; }
 };
 
-// y = act(conv3x3x3(x, w) + bias); w packed (pack_weights); relu: 0/1; bias may be nullptr.
-cudaError_t conv_fwd(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout, int relu,
-                     cudaStream_t st);
-// The same convolution on the tcgen05 tensor cores (net_tc.cu): M = 128 voxels per CTA,
-// accumulator in tensor memory.
-cudaError_t conv_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout, int relu,
-                        cudaStream_t st);
+// y = act(conv3x3x3(x, w) + bias); w packed (pack_weights); relu: 0/1; bias may be nullptr; mask
+// (may be nullptr): an activation of y's shape, y is zero where it is not positive.  On the
+// tcgen05 tensor cores (net_tc.cu): M = 128 voxels per slice, accumulator in tensor memory.
+cudaError_t conv_fwd(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask, bf16 *y, Vol v, int cin,
+                     int cout, int relu, cudaStream_t st);
 // The tcgen05 convolution's error word (0, or 1 after a bounded wait ran out); synchronises
 // the stream; reset: clear it after reading.
 cudaError_t conv_tc_error(unsigned *err, bool reset, cudaStream_t st);
@@ -43,24 +41,24 @@ cudaError_t bias_grad(const bf16 *dy, float *db, long long voxels, int c, cudaSt
 long long packed_weights(int cin, int cout);
 cudaError_t pack_weights(const float *w, bf16 *out, int cin, int cout, bool flip, cudaStream_t st);
 
-// elementwise and resampling (channels-last, c channels)
-cudaError_t relu_bwd(const bf16 *y, bf16 *dy, long long n, cudaStream_t st);      // dy *= (y > 0)
-cudaError_t add_into(bf16 *a, const bf16 *b, long long n, cudaStream_t st);       // a += b
+// Resampling (channels-last, c channels; `fine` the volume at the finer level).
 cudaError_t pool_fwd(const bf16 *x, bf16 *y, Vol fine, int c, cudaStream_t st);   // 2x2x2 mean
-cudaError_t pool_bwd(const bf16 *dy, bf16 *dx, Vol fine, int c, cudaStream_t st);
-cudaError_t up_fwd(const bf16 *x, bf16 *y, Vol fine, int c, cudaStream_t st);     // nearest x2
-cudaError_t up_bwd(const bf16 *dy, bf16 *dx, Vol fine, int c, cudaStream_t st);
-cudaError_t concat_fwd(const bf16 *a, int ca, const bf16 *b, int cb, bf16 *y, long long voxels, cudaStream_t st);
-cudaError_t concat_bwd(const bf16 *dy, bf16 *da, int ca, bf16 *db, int cb, long long voxels, cudaStream_t st);
+// y = [x (ca channels) nearest-upsampled x2 | skip (cb)]
+cudaError_t up_concat(const bf16 *x, int ca, const bf16 *skip, int cb, bf16 *y, Vol fine, cudaStream_t st);
+// Their gradients through the ReLU that made x, from the gradient dy of a concatenation of c
+// channels: dx of the upsampled half (the first ca), and of the skip half (the last cb) with the
+// pooling path's gradient dp added.
+cudaError_t up_bwd(const bf16 *dy, int c, const bf16 *x, bf16 *dx, int ca, Vol fine, cudaStream_t st);
+cudaError_t skip_bwd(const bf16 *dy, int c, const bf16 *dp, const bf16 *x, bf16 *dx, int cb, Vol fine, cudaStream_t st);
 
-// Head: tau[v] = 1 + sum_c wh[c] y[v][c] + bh[0].  With a target (target[v] > 0 marks the
-// voxels of the loss), acc[0] += sum (tau - target)^2 and acc[1] += count.
+// Head: tau[v] = 1 + sum_c wh[c] y[v][c] + bh[0], 16 channels.  With a target (target[v] > 0 marks
+// the voxels of the loss), acc[0] += sum (tau - target)^2 and acc[1] += count.
 cudaError_t head_fwd(const bf16 *y, const float *wh, const float *bh, float *tau, const float *target, long long voxels,
-                     int c, double *acc, cudaStream_t st);
-// Gradients of loss = acc[0] / acc[1]: dy[v][c] = g wh[c], dwh[c] += sum g y[v][c],
+                     double *acc, cudaStream_t st);
+// Gradients of loss = acc[0] / acc[1]: dy[v][c] = relu'(y[v][c]) g wh[c], dwh[c] += sum g y[v][c],
 // dbh += sum g, with g = 2 (tau - target) / acc[1] on the loss voxels, else 0.
 cudaError_t head_bwd(const bf16 *y, const float *wh, const float *tau, const float *target, const double *acc, bf16 *dy,
-                     float *dwh, float *dbh, long long voxels, int c, cudaStream_t st);
+                     float *dwh, float *dbh, long long voxels, cudaStream_t st);
 
 // Adam on n FP32 parameters (bias-corrected, step t >= 1)
 cudaError_t adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,

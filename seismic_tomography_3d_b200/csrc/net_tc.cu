@@ -138,8 +138,8 @@ __device__ __forceinline__ TcTile tc_tile(long long t, const Vol &v)
 }
 
 template <int NT, int DS>
-__global__ void __launch_bounds__(128) k_conv_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, bf16 *y,
-                                                     Vol v, int cin, int cout, int relu)
+__global__ void __launch_bounds__(128) k_conv_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask,
+                                                     bf16 *y, Vol v, int cin, int cout, int relu)
 {
     constexpr unsigned kWeightBytes = weight_bytes(NT);
     constexpr unsigned kHalfBytes = half_bytes(DS);
@@ -269,6 +269,11 @@ __global__ void __launch_bounds__(128) k_conv_fwd_tc(const bf16 *x, const bf16 *
             tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(sl * NT + c), acc);
             if (!inside || co0 + c >= cout) continue;
             uint32_t packed[8];
+            uint4 gate[2];
+            if (mask) {
+                gate[0] = __ldg(reinterpret_cast<const uint4 *>(mask + vox * cout + co0 + c));
+                gate[1] = __ldg(reinterpret_cast<const uint4 *>(mask + vox * cout + co0 + c) + 1);
+            }
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 float v0 = acc[2 * j], v1 = acc[2 * j + 1];
@@ -279,6 +284,11 @@ __global__ void __launch_bounds__(128) k_conv_fwd_tc(const bf16 *x, const bf16 *
                 if (relu) {
                     v0 = fmaxf(v0, 0.f);
                     v1 = fmaxf(v1, 0.f);
+                }
+                if (mask) {
+                    const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 *>(gate)[j]);
+                    v0 = f.x > 0.f ? v0 : 0.f;
+                    v1 = f.y > 0.f ? v1 : 0.f;
                 }
                 const __nv_bfloat162 p2 = __floats2bfloat162_rn(v0, v1);
                 packed[j] = *reinterpret_cast<const uint32_t *>(&p2);
@@ -297,14 +307,14 @@ __global__ void __launch_bounds__(128) k_conv_fwd_tc(const bf16 *x, const bf16 *
 }
 
 template <int NT, int DS>
-cudaError_t launch_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout, int relu,
-                          long long tiles, cudaStream_t st)
+cudaError_t launch_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask, bf16 *y, Vol v, int cin,
+                          int cout, int relu, long long tiles, cudaStream_t st)
 {
     const size_t smem = 2 * (size_t)half_bytes(DS) + weight_bytes(NT) + 32;
     cudaError_t e = cudaFuncSetAttribute(k_conv_fwd_tc<NT, DS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)tiles, (unsigned)((cout + NT - 1) / NT));
-    k_conv_fwd_tc<NT, DS><<<grid, 128, smem, st>>>(x, w, bias, y, v, cin, cout, relu);
+    k_conv_fwd_tc<NT, DS><<<grid, 128, smem, st>>>(x, w, bias, mask, y, v, cin, cout, relu);
     return cudaGetLastError();
 }
 
@@ -320,18 +330,18 @@ int tc_columns(int cout) { return cout <= 64 || cout == 80 ? cout : 64; }
 // Slices per CTA: as many as keep about two CTAs per SM busy (more slices share one weight
 // staging and each A tile; fewer give small volumes enough CTAs).
 template <int NT>
-cudaError_t launch_fwd_tc_ds(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout,
-                             int relu, cudaStream_t st)
+cudaError_t launch_fwd_tc_ds(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask, bf16 *y, Vol v, int cin,
+                             int cout, int relu, cudaStream_t st)
 {
     const long long chunks = (cout + NT - 1) / NT, want = 2LL * 148;
     if (tc_tiles(v, 1) >= (1LL << 31)) return cudaErrorInvalidValue;
     constexpr int kBig = NT <= 32 ? 8 : 4, kMid = NT <= 64 ? 4 : 2;
     if (NT <= 32 && tc_tiles(v, kBig) * chunks >= 2 * want)
-        return launch_fwd_tc<NT, kBig>(x, w, bias, y, v, cin, cout, relu, tc_tiles(v, kBig), st);
+        return launch_fwd_tc<NT, kBig>(x, w, bias, mask, y, v, cin, cout, relu, tc_tiles(v, kBig), st);
     if (tc_tiles(v, kMid) * chunks >= want)
-        return launch_fwd_tc<NT, kMid>(x, w, bias, y, v, cin, cout, relu, tc_tiles(v, kMid), st);
-    if (tc_tiles(v, 2) * chunks >= want) return launch_fwd_tc<NT, 2>(x, w, bias, y, v, cin, cout, relu, tc_tiles(v, 2), st);
-    return launch_fwd_tc<NT, 1>(x, w, bias, y, v, cin, cout, relu, tc_tiles(v, 1), st);
+        return launch_fwd_tc<NT, kMid>(x, w, bias, mask, y, v, cin, cout, relu, tc_tiles(v, kMid), st);
+    if (tc_tiles(v, 2) * chunks >= want) return launch_fwd_tc<NT, 2>(x, w, bias, mask, y, v, cin, cout, relu, tc_tiles(v, 2), st);
+    return launch_fwd_tc<NT, 1>(x, w, bias, mask, y, v, cin, cout, relu, tc_tiles(v, 1), st);
 }
 
 // Element e of a convolution's packed weights (weight_bytes): the convolution with weights
@@ -362,16 +372,16 @@ __global__ void k_pack_weights(const float *w, bf16 *out, int cin, int cout, int
 
 }  // namespace
 
-cudaError_t conv_fwd_tc(const bf16 *x, const bf16 *w, const float *bias, bf16 *y, Vol v, int cin, int cout, int relu,
-                        cudaStream_t st)
+cudaError_t conv_fwd(const bf16 *x, const bf16 *w, const float *bias, const bf16 *mask, bf16 *y, Vol v, int cin,
+                     int cout, int relu, cudaStream_t st)
 {
     if (cin % 16 || cout % 16 || cin < 16 || cout < 16) return cudaErrorInvalidValue;
     switch (tc_columns(cout)) {
-    case 16: return launch_fwd_tc_ds<16>(x, w, bias, y, v, cin, cout, relu, st);
-    case 32: return launch_fwd_tc_ds<32>(x, w, bias, y, v, cin, cout, relu, st);
-    case 48: return launch_fwd_tc_ds<48>(x, w, bias, y, v, cin, cout, relu, st);
-    case 80: return launch_fwd_tc_ds<80>(x, w, bias, y, v, cin, cout, relu, st);
-    default: return launch_fwd_tc_ds<64>(x, w, bias, y, v, cin, cout, relu, st);
+    case 16: return launch_fwd_tc_ds<16>(x, w, bias, mask, y, v, cin, cout, relu, st);
+    case 32: return launch_fwd_tc_ds<32>(x, w, bias, mask, y, v, cin, cout, relu, st);
+    case 48: return launch_fwd_tc_ds<48>(x, w, bias, mask, y, v, cin, cout, relu, st);
+    case 80: return launch_fwd_tc_ds<80>(x, w, bias, mask, y, v, cin, cout, relu, st);
+    default: return launch_fwd_tc_ds<64>(x, w, bias, mask, y, v, cin, cout, relu, st);
     }
 }
 
