@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "common.cuh"
 #include "net.cuh"
 
 namespace tomo {
@@ -533,8 +534,9 @@ __device__ __forceinline__ void axis_weight(int x, int k, int n, int &c0, int &c
 // counter instead of a division), and the values interpolated along z are reloaded only
 // where x enters a new cell.  Lanes follow z, the fastest axis, across column ends, so no
 // lane idles on a depth that is not a multiple of 32.  64 windows of 201 x 201 x 101 at
-// stride 4 (261 M nodes): the kernel 3.70 -> 0.7 ms, the whole prediction 7.49 -> 4.50 ms.
-constexpr int kTimeRun = 32;
+// stride 4 (261 M nodes): the kernel 3.70 -> 0.52 ms (0.71 with IEEE root and
+// division and runs of 32), 83 % of the issue slots.
+constexpr int kTimeRun = 64;
 
 template <bool kStrided>
 __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, const float *tau, float *t_out)
@@ -569,7 +571,7 @@ __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, c
         float *out = t_out + j.nat_off + z + (long long)j.nz * (xa + (long long)j.wnx * y);
         int c = xa / k, rem = xa - c * k;  // x = c k + rem
         int c1 = min(c + 1, nc - 1);
-        float den = (float)(min(c1 * k, j.wnx - 1) - c * k);
+        Divisor den = divisor((float)(min(c1 * k, j.wnx - 1) - c * k));
         float c00 = 0.f, c01 = 0.f, c10 = 0.f, c11 = 0.f;
         if (kStrided) {
             c00 = at(p00, p10, c);
@@ -582,7 +584,7 @@ __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, c
                 rem = 0;
                 c = c1;
                 c1 = min(c + 1, nc - 1);
-                den = (float)(min(c1 * k, j.wnx - 1) - c * k);
+                den = divisor((float)(min(c1 * k, j.wnx - 1) - c * k));
                 c00 = c10;
                 c01 = c11;
                 if (c1 > c) {
@@ -591,11 +593,11 @@ __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, c
                 }
             }
             const float ex = x * h - j.sx;
-            const float dist = sqrtf(ex * ex + ey * ey + ez * ez);
+            const float dist = fsqrt(ex * ex + ey * ey + ez * ez);
             float t = 0.f;
             if (dist >= h) {
                 if (kStrided) {
-                    const float tx = den > 0.f ? (float)rem / den : 0.f;
+                    const float tx = den.y > 0.f ? fdiv((float)rem, den) : 0.f;
                     const float c0 = c00 * (1.f - tx) + c10 * tx, cc = c01 * (1.f - tx) + c11 * tx;
                     t = (c0 * (1.f - ty) + cc * ty) * s_src * dist;
                 } else {
