@@ -184,6 +184,7 @@ extern "C" int tomo_iteration(tomo_ctx *ctx, int nshots, const tomo_point *shots
                           (const void *)ctx->shots_d.ptr, (const void *)ctx->rec.ptr, (const void *)ctx->qflag8.ptr})
         push(key_a, p);
     push(key_a, plan.brick8);
+    push(key_a, plan.cluster);
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if (graphs && (!G.a || key_a != G.key_a)) {
         if (G.a) cudaGraphExecDestroy(G.a);

@@ -96,6 +96,7 @@ struct tomo_ctx {
     int nshots = 0, nrec = 0;
     bool have_solve = false;
     // launch shape chosen by tomo_eik_autotune (0: not tuned)
+    int cluster_bricks = 0;       // largest shot one cluster can hold (fim_cluster_limit)
     int tuned_block_warps = 0, tuned_occupancy = 0, tuned_max_inner = 0;
     int tuned_brick = 0;          // 0: none chosen (4^3); TOMO_BRICK_4 / TOMO_BRICK_8
     int tuned_schedule = 0;       // 0: none chosen (rounds); TOMO_SCHED_PAIR

@@ -18,6 +18,8 @@
 //    ahead of its shot's front waits on a parking list: rounds then follow traveltime
 //    rather than brick-graph distance, which removes the re-activation cascades of smooth
 //    v(z) models.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "fim.cuh"
 
@@ -147,13 +149,12 @@ __device__ __forceinline__ void gather_S2(const float *S, int gbx, int gbz, cons
 // from the floor node of the window-cropped field, with the reference's flattened index
 // arithmetic (an offset past a column wraps into the next; past the end: 0).  Grid-stride
 // over (shot, receiver); receivers outside a shot's window get kInf.
-__device__ void sample_receivers(const float *T, const ShotDesc *shots, int nshots, const float *rx,
-                                 const float *ry, const float *rz, int nrec, float dx, float dy, float dz,
-                                 int nz_, float *t_recv)
+// (sample_range: entries first, first + stride, ... below end of the shot x receiver table.)
+__device__ void sample_range(const float *T, const ShotDesc *shots, const float *rx, const float *ry, const float *rz,
+                             int nrec, float dx, float dy, float dz, int nz_, float *t_recv, long long first,
+                             long long end, long long stride)
 {
-    const long long total = (long long)nshots * nrec;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
+    for (long long e = first; e < end; e += stride) {
         const int s = (int)(e / nrec), r = (int)(e % nrec);
         const ShotDesc &d = shots[s];
         const float x = fsub(rx[r], fmul((float)d.wx0, dx));
@@ -185,6 +186,14 @@ __device__ void sample_receivers(const float *T, const ShotDesc *shots, int nsho
         }
         t_recv[e] = trilinear_ref(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], x0, x1, y0, y1, z0, z1, x, y, z);
     }
+}
+
+__device__ void sample_receivers(const float *T, const ShotDesc *shots, int nshots, const float *rx,
+                                 const float *ry, const float *rz, int nrec, float dx, float dy, float dz,
+                                 int nz_, float *t_recv)
+{
+    sample_range(T, shots, rx, ry, rz, nrec, dx, dy, dz, nz_, t_recv, blockIdx.x * (long long)blockDim.x + threadIdx.x,
+                 (long long)nshots * nrec, (long long)gridDim.x * blockDim.x);
 }
 
 struct WarpStats {
@@ -742,6 +751,272 @@ __global__ void __launch_bounds__(512) __maxnreg__(fim_regs(MINB)) k_fim_solve(F
     if (!ok || p.nrec == 0) return;
 
     sample_receivers(p.T, p.shots, p.nshots, p.rx, p.ry, p.rz, p.nrec, p.dx, p.dy, p.dz, p.nz, p.t_recv);
+}
+
+// ---------------------------------------------------------------------------------------
+// Small batches: one shot per thread-block cluster, its whole field in the cluster's shared
+// memory (FimLaunch of a batch whose shots each fit, fim_cluster_fits).
+//
+// A shot of a few thousand bricks has tens to hundreds of them to relax in a round, so a round
+// of k_fim_solve lasts as long as its chain of dependent accesses to L2 -- list count, item,
+// traveltimes, queue flag, list slot -- and the grid barrier after them: 6.8 us, of which the
+// relaxation is a fifth, and 8.9 us where 296 CTAs arrive at the barrier for 250 bricks.
+// Here a brick belongs to one CTA of the cluster (cluster_owner), which keeps its 64 traveltimes and a bit
+// "relax in the next round" in shared memory.  Neighbours' faces are read through distributed
+// shared memory; queueing a brick sets its owner's bit, a reduction nobody waits for (flags,
+// counts and lists as in k_fim_solve cost two round trips more at the end of an item); a round
+// ends at the hardware's cluster barrier, every warp finds the CTA's bricks of the round in the
+// 24 words of its bit map, and the field is written to the pool once, at the end.  Rounds, in-brick relaxation,
+// queueing tests and tolerances are those of k_fim_solve.  Clusters do not wait for each other
+// (no cooperative launch).  ms per call, against one grid of 148 CTAs: 360 bricks 0.134 | 0.175 (1 to
+// 4 shots alike), 1,000 0.176 | 0.258, 3,375 0.232 | 0.298, 8,788 0.370 | 0.391.
+// ---------------------------------------------------------------------------------------
+constexpr int kClusterWarps = 16;
+
+// Shared memory of one CTA with room for `cap` bricks.
+constexpr size_t cluster_smem(int cap)
+{
+    return ((size_t)cap * kBrickNodes + kClusterWarps * kTileNodes) * sizeof(float) + (3 * 32 + 6) * sizeof(unsigned);
+}
+constexpr int kClusterMaxCap = 32 * 32;  // a bit map is one word per lane
+
+// Distributed shared memory: the address of this CTA's `local` in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned cluster_addr(const void *local, unsigned rank)
+{
+    unsigned a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float cluster_load(unsigned a)
+{
+    float v;
+    asm volatile("ld.relaxed.cluster.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_or(unsigned a, unsigned v)
+{
+    asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Owner of brick b: the 16 bricks of a group q = b / 16 go to the 16 CTAs in an order that a hash
+// of q turns, so that a wavefront, whose bricks differ by a few fixed strides, spreads evenly.
+// (16 is the largest cluster, an opt-in size; 8, the portable one: 0.141 vs 0.136 ms on 360 bricks,
+// and half the capacity.)
+constexpr unsigned kClusterCtas = 16;
+__device__ __forceinline__ unsigned cluster_turn(unsigned q) { return (q * 0x9E3779B1u) >> 28; }
+__device__ __forceinline__ unsigned cluster_owner(unsigned b) { return (b + cluster_turn(b / kClusterCtas)) % kClusterCtas; }
+__device__ __forceinline__ unsigned cluster_brick(unsigned rank, unsigned q)
+{
+    return q * kClusterCtas + (rank - cluster_turn(q)) % kClusterCtas;
+}
+
+// Position of the k-th (from 0) set bit of m, which has more than k.
+__device__ __forceinline__ unsigned nth_bit(unsigned m, unsigned k)
+{
+    unsigned at = 0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+        const unsigned below = (unsigned)__popc(m & ((1u << w) - 1u));
+        if (k >= below) {
+            k -= below;
+            m >>= w;
+            at += w;
+        }
+    }
+    return at;
+}
+
+template <bool kFastSqrt, bool kGather>
+__global__ void __launch_bounds__(32 * kClusterWarps, 1) k_fim_cluster(FimLaunch p, int cap)
+{
+    namespace cg = cooperative_groups;
+    const cg::cluster_group cluster = cg::this_cluster();
+    constexpr unsigned C = kClusterCtas;
+    const unsigned rank = cluster.block_rank();
+    const int s = (int)(blockIdx.x / C);
+    const ShotDesc d = p.shots[s];  // a copy: its fields would be read again after every store
+    const int nbz = d.nbz, nbx = d.nbx, nby = d.nby;
+    const unsigned nb = (unsigned)nbz * nbx * nby;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ float smem[];
+    float *T = smem;                                              // cap x 64 traveltimes
+    float *tile = T + (size_t)cap * kBrickNodes + warp * kTileNodes;
+    // bit maps of three rotating rounds (32 words each), per round whether this CTA set any bit, and
+    // the cursors over a round's bricks
+    unsigned *bits = reinterpret_cast<unsigned *>(T + (size_t)cap * kBrickNodes + kClusterWarps * kTileNodes);
+    volatile unsigned *any = bits + 3 * 32;
+    unsigned *cursor = bits + 3 * 32 + 3;
+
+    const unsigned mine = (nb + C - 1) / C;  // this CTA's bricks (the last of them may lie past nb)
+    for (unsigned i = threadIdx.x; i < mine * kBrickNodes; i += blockDim.x) T[i] = kInf;
+    if (threadIdx.x < 3 * 32 + 6) bits[threadIdx.x] = 0u;
+    __syncthreads();
+    const unsigned src = (unsigned)d.src_brick;
+    if (threadIdx.x == 0 && cluster_owner(src) == rank) {  // as k_fim_seed
+        int bz, bx, by;
+        brick_coords(d, src, bz, bx, by);
+        T[src / C * kBrickNodes + d.src_node] =
+            __fmul_rn(node_S(p.S, p.gbx, p.gbz, d, bz, bx, by, d.src_node), d.src_dist);
+        bits[src / C / 32u] = 1u << (src / C % 32u);
+        any[0] = 1u;
+    }
+    cluster.sync();
+
+    const int z0 = lane & 3, x0 = (lane >> 2) & 3, y0 = 2 * (lane >> 4), n0 = lane_node(lane);
+    const int ti0 = tile_idx(z0, x0, y0), ti1 = ti0 + kTileY;
+    const bool red0 = ((z0 + x0) & 1) == 0;
+    const int tA = red0 ? ti0 : ti1, tB = red0 ? ti1 : ti0, yA = red0 ? -kTileY : kTileY;
+    WarpStats ws{0ull, 0ull, 0ull, 0ull};
+    unsigned round = 0;
+    for (;; ++round) {
+        const unsigned cur = round % 3u;
+        // whether any CTA has work: final at the last barrier, reset two rounds on
+        const unsigned c = (unsigned)lane < C ? __float_as_uint(cluster_load(cluster_addr(bits + 3 * 32 + cur, lane))) : 0u;
+        if (!__any_sync(kFull, c != 0u)) break;
+        if ((int)round >= p.max_rounds) {
+            if (threadIdx.x == 0) atomicCAS(p.ctrl + kErr, 0u, (unsigned)kDevRoundCap);
+            break;
+        }
+        if (threadIdx.x < 32) bits[(round + 2u) % 3u * 32u + threadIdx.x] = 0u;
+        if (threadIdx.x == 0) any[(round + 2u) % 3u] = cursor[(round + 2u) % 3u] = 0u;
+        // the CTA's bricks of this round: the set bits, in order
+        const unsigned word = bits[cur * 32u + lane];
+        unsigned through = (unsigned)__popc(word);  // set bits up to and including this lane's word
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(kFull, through, o);
+            if (lane >= o) through += v;
+        }
+        const unsigned n = __shfl_sync(kFull, through, 31), before = through - (unsigned)__popc(word);
+        const unsigned nxt = (round + 1u) % 3u;
+        for (unsigned i = warp; i < n;) {
+            const int holder = __ffs(__ballot_sync(kFull, through > i)) - 1;
+            const unsigned at = 32u * holder + nth_bit(__shfl_sync(kFull, word, holder),
+                                                       i - __shfl_sync(kFull, before, holder));
+            const unsigned b = cluster_brick(rank, at);
+            int bz, bx, by;
+            brick_coords(d, b, bz, bx, by);
+            // ---- load ----
+            float s0, s1;
+            if (!kGather || !d.s_gather) {
+                const float *Sb = model_brick_S(p.S, p.gbx, p.gbz, d, bz, bx, by);
+                s0 = __ldg(Sb + n0);
+                s1 = __ldg(Sb + n0 + 16);
+            } else {
+                gather_S2(p.S, p.gbx, p.gbz, d, bz, bx, by, n0, s0, s1);
+            }
+            volatile float *Tb = T + (size_t)at * kBrickNodes;
+            const float i0 = Tb[n0], i1 = Tb[n0 + 16];
+            float hv[3];
+            int ht[3];
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                int node;
+                const long long to = halo_slot(d, b, bz, bx, by, lane, q, node, ht[q]);
+                hv[q] = kInf;
+                if (to >= 0)
+                    hv[q] = cluster_load(cluster_addr(T, cluster_owner((unsigned)to)) +
+                                         ((unsigned)to / C * kBrickNodes + node) * (unsigned)sizeof(float));
+            }
+            tile[ti0] = i0;
+            tile[ti1] = i1;
+#pragma unroll
+            for (int q = 0; q < 3; q++) tile[ht[q]] = hv[q];
+            __syncwarp();
+            // ---- red-black relaxation (relax_brick) ----
+            float cA = red0 ? i0 : i1, cB = red0 ? i1 : i0;
+            const NodeConst kA = node_const(p.h, red0 ? s0 : s1), kB = node_const(p.h, red0 ? s1 : s0);
+            bool more = true;
+            int it = 0;
+            for (; it < p.max_inner; ++it) {
+                const float aA = fminf(tile[tA - kTileX], tile[tA + kTileX]);
+                const float gA = fminf(tile[tA - 1], tile[tA + 1]);
+                const float bA = fminf(tile[tA + yA], cB);
+                const float nA = fminf(cA, godunov_jw<kFastSqrt, false>(aA, bA, gA, kA));
+                tile[tA] = nA;
+                const bool chA = nA < cA - p.inner_tol;
+                cA = nA;
+                __syncwarp();
+                if (it > 0 && !__any_sync(kFull, chA)) {
+                    more = false;
+                    ++it;
+                    break;
+                }
+                const float aB = fminf(tile[tB - kTileX], tile[tB + kTileX]);
+                const float gB = fminf(tile[tB - 1], tile[tB + 1]);
+                const float bB = fminf(tile[tB - yA], nA);
+                const float nB = fminf(cB, godunov_jw<kFastSqrt, false>(aB, bB, gB, kB));
+                tile[tB] = nB;
+                const bool chB = nB < cB - p.inner_tol;
+                cB = nB;
+                __syncwarp();
+                if (!__any_sync(kFull, chB)) {
+                    more = false;
+                    ++it;
+                    break;
+                }
+            }
+            // ---- store, face tests, queueing ----
+            const float c0 = red0 ? cA : cB, c1 = red0 ? cB : cA;
+            const bool any_drop = __any_sync(kFull, (c0 < i0) | (c1 < i1));
+            if (any_drop) {
+                Tb[n0] = c0;
+                Tb[n0 + 16] = c1;
+            }
+            ws.act += 1;
+            ws.inner += (unsigned long long)it;
+            if (!any_drop) ws.idle += 1;
+            const bool d0 = c0 < i0 - p.change_tol, d1 = c1 < i1 - p.change_tol;
+            unsigned fl = 0;  // faces: 1 z-, 2 z+, 4 x-, 8 x+, 16 y-, 32 y+
+            if (z0 == 0 && ((d0 && c0 < tile[ti0 - 1]) || (d1 && c1 < tile[ti1 - 1]))) fl |= 1u;
+            if (z0 == 3 && ((d0 && c0 < tile[ti0 + 1]) || (d1 && c1 < tile[ti1 + 1]))) fl |= 2u;
+            if (x0 == 0 && ((d0 && c0 < tile[ti0 - kTileX]) || (d1 && c1 < tile[ti1 - kTileX]))) fl |= 4u;
+            if (x0 == 3 && ((d0 && c0 < tile[ti0 + kTileX]) || (d1 && c1 < tile[ti1 + kTileX]))) fl |= 8u;
+            if (y0 == 0 && d0 && c0 < tile[ti0 - kTileY]) fl |= 16u;
+            if (y0 == 2 && d1 && c1 < tile[ti1 + kTileY]) fl |= 32u;
+            const unsigned face = __reduce_or_sync(kFull, fl);
+            bool want = false;
+            int tgt = (int)b;
+            if (lane < 6) {
+                const int axis = lane >> 1;
+                const bool up = lane & 1;
+                const int cc = axis == 0 ? bz : (axis == 1 ? bx : by);
+                const int nmax = axis == 0 ? nbz : (axis == 1 ? nbx : nby);
+                const int stride = axis == 0 ? 1 : (axis == 1 ? nbz : nbz * nbx);
+                want = ((face >> lane) & 1u) && (up ? cc < nmax - 1 : cc > 0);
+                tgt += up ? stride : -stride;
+            } else if (lane == 6) {
+                want = more;
+            }
+            if (want) {
+                const unsigned owner = cluster_owner((unsigned)tgt), to = (unsigned)tgt / C;
+                cluster_or(cluster_addr(bits + nxt * 32u + to / 32u, owner), 1u << (to % 32u));
+                any[nxt] = 1u;  // here, wherever the brick lives: there is a next round
+            }
+            if (lane == 0) i = kClusterWarps + atomicAdd(cursor + cur, 1u);
+            i = __shfl_sync(kFull, i, 0);  // (and the tile is free for the next item)
+        }
+        cluster.sync();
+    }
+    if (lane == 0 && ws.act) {
+        atomicAdd(p.stats + 0, ws.act);
+        atomicAdd(p.stats + 1, ws.inner);
+        atomicAdd(p.stats + 3, ws.idle);
+    }
+    if (rank == 0 && threadIdx.x == 0) atomicMax(p.ctrl + kRounds, round);
+    // the field into the pool, for the receivers and whoever reads it later
+    float4 *pool = reinterpret_cast<float4 *>(p.T + d.t_off);
+    const float4 *T4 = reinterpret_cast<const float4 *>(T);
+    for (unsigned i = threadIdx.x; i < mine * (kBrickNodes / 4); i += blockDim.x) {
+        const unsigned b = cluster_brick(rank, i / 16u);
+        if (b < nb) __stcg(pool + (size_t)b * 16u + i % 16u, T4[i]);
+    }
+    __threadfence();
+    cluster.sync();  // also: nobody reads this CTA's words any more
+    if (p.nrec)
+        sample_range(p.T, p.shots, p.rx, p.ry, p.rz, p.nrec, p.dx, p.dy, p.dz, p.nz, p.t_recv,
+                     (long long)s * p.nrec + rank * blockDim.x + threadIdx.x, (long long)(s + 1) * p.nrec,
+                     (long long)C * blockDim.x);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -2004,7 +2279,12 @@ static cudaError_t launch_solve(const FimLaunch &p, int block_warps, bool async,
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int grid = nsm * per_sm;
+    // Few bricks: one CTA per SM, since a round then lasts as long as its chain of accesses and its
+    // barrier, which half the CTAs reach sooner.  ms per call, one | two: 1 shot of 3,375 bricks 0.31 |
+    // 0.36, of 8,788 0.40 | 0.49, of 66,300 0.84 | 0.95, 2 of them 0.99 | 1.05; but 4 of them 1.39 | 1.33,
+    // 16 of 8,788 0.78 | 0.78.
+    const bool few = !async && block_warps >= 16 && p.list_cap <= 131072u;
+    const int grid = nsm * (few ? 1 : per_sm);
     if (grid_out) *grid_out = grid;
     FimLaunch pp = p;
     void *args[] = {&pp};
@@ -2031,6 +2311,50 @@ cudaError_t fim_solve(const FimLaunch &p, int block_warps, int occupancy, bool i
     if (block_warps < 1 || block_warps > 16) block_warps = 16;
     return ieee_sqrt ? solve_occ<false>(p, block_warps, occupancy, async, grid_out, st)
                      : solve_occ<true>(p, block_warps, occupancy, async, grid_out, st);
+}
+
+
+static const void *cluster_kernel(bool ieee_sqrt, bool gather)
+{
+    return ieee_sqrt ? (gather ? (const void *)k_fim_cluster<false, true> : (const void *)k_fim_cluster<false, false>)
+                     : (gather ? (const void *)k_fim_cluster<true, true> : (const void *)k_fim_cluster<true, false>);
+}
+
+cudaError_t fim_cluster_limit(int *max_bricks)
+{
+    *max_bricks = 0;
+    int dev = 0, smem = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    int cap = 0;
+    while (cap < kClusterMaxCap && cluster_smem(cap + 1) <= (size_t)smem) cap++;
+    *max_bricks = cap * (int)kClusterCtas;
+    return cudaSuccess;
+}
+
+cudaError_t fim_solve_cluster(const FimLaunch &p, long long max_bricks, bool ieee_sqrt, cudaStream_t st)
+{
+    const int cap = (int)((max_bricks + (int)kClusterCtas - 1) / (int)kClusterCtas);
+    const void *fn = cluster_kernel(ieee_sqrt, p.gather != 0);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(cap));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kClusterCtas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kClusterCtas * (unsigned)p.nshots);
+    cfg.blockDim = dim3(32 * kClusterWarps);
+    cfg.dynamicSmemBytes = cluster_smem(cap);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    FimLaunch pp = p;
+    int c = cap;
+    void *args[] = {&pp, &c};
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 template <int MINB, bool kFastSqrt>

@@ -35,6 +35,7 @@ struct EikPlan {
     FimLaunch p;
     int block_warps, occupancy;
     bool ieee_sqrt, async, brick8;
+    long long cluster;  // bricks of the largest shot if each solves in a cluster, else 0
     size_t t_total, q_total;
 };
 int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_window *windows, int nrec,
