@@ -154,6 +154,7 @@ void tomo_release_tomography(tomo_ctx *ctx)
                     &ctx->vel_out, &ctx->gauss_kernel})
         b->release();
     ctx->runs.release();
+    ctx->ray_counts.release();
     ctx->cub_temp.release();
     ctx->partials.release();
     ctx->hist.release();
@@ -374,10 +375,12 @@ int tomo_build_jacobian(tomo_ctx *ctx, const tomo_jacobian_opts *opts, tomo_jaco
     if (rc != TOMO_OK) return rc;
     CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     const long long nrays = jg.nrays;
-    std::vector<int> st((size_t)nrays), steps((size_t)nrays);
-    CK(cudaMemcpyAsync(st.data(), ctx->ray_status.ptr, st.size() * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(steps.data(), ctx->ray_steps.ptr, steps.size() * sizeof(int), cudaMemcpyDeviceToHost,
-                       ctx->stream));
+    unsigned long long cnt[tomo::kRayCounts] = {};
+    if (stats) {
+        CK(ctx->ray_counts.ensure(tomo::kRayCounts));
+        CK(tomo::ray_stats(ctx->ray_status.ptr, ctx->ray_steps.ptr, (int)nrays, ctx->ray_counts.ptr, ctx->stream));
+        CK(cudaMemcpyAsync(cnt, ctx->ray_counts.ptr, sizeof(cnt), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     tomo::jac_commit(ctx, jg, nnz_g, nnz);
     if (stats) {
@@ -390,17 +393,13 @@ int tomo_build_jacobian(tomo_ctx *ctx, const tomo_jacobian_opts *opts, tomo_jaco
         stats->nnz_rays = nnz_g;
         stats->nnz = nnz;
         stats->rays = nrays;
-        long long cnt[6] = {0, 0, 0, 0, 0, 0};
-        for (size_t i = 0; i < st.size(); i++) {
-            if (st[i] >= 0 && st[i] < 6) cnt[st[i]]++;
-            stats->ray_steps += steps[i];
-        }
-        stats->rays_ok = cnt[0];
-        stats->rays_stalled = cnt[1];
-        stats->rays_capped = cnt[2];
-        stats->rays_nonfinite = cnt[3];
-        stats->rays_outside = cnt[4];
-        stats->rays_overflow = cnt[5];
+        stats->rays_ok = (long long)cnt[0];
+        stats->rays_stalled = (long long)cnt[1];
+        stats->rays_capped = (long long)cnt[2];
+        stats->rays_nonfinite = (long long)cnt[3];
+        stats->rays_outside = (long long)cnt[4];
+        stats->rays_overflow = (long long)cnt[5];
+        stats->ray_steps = (long long)cnt[6];
         cudaEventElapsedTime(&stats->ms, ctx->ev[0], ctx->ev[1]);
     }
     return TOMO_OK;

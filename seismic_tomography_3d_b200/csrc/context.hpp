@@ -109,6 +109,7 @@ struct tomo_ctx {
     // ray tracing scratch
     tomo::DevBuf<uint2> runs;
     tomo::DevBuf<int> nuniq, ray_status, ray_steps;
+    tomo::DevBuf<unsigned long long> ray_counts;
     tomo::DevBuf<float> final_dist, spos, tk_coef, illum;
     // A = [G ; lambda L] in CSR and its transpose
     tomo::DevBuf<int> a_ptr, a_idx, t_ptr, t_idx;

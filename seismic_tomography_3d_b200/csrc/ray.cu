@@ -310,6 +310,29 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_ray_sort(RayLaunch p)
     }
 }
 
+// Rays per status and their steps: counts[0..5], counts[6].  (Copying both arrays to pageable host
+// memory and counting there took 0.35 ms for 160,000 rays.)
+__global__ void __launch_bounds__(256) k_ray_stats(const int *status, const int *steps, int nrays,
+                                                   unsigned long long *counts)
+{
+    __shared__ unsigned long long sh[7];
+    if (threadIdx.x < 7) sh[threadIdx.x] = 0ull;
+    __syncthreads();
+    unsigned long long total = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i - (int)(threadIdx.x & 31) < nrays; i += gridDim.x * blockDim.x) {
+        const int st = i < nrays ? status[i] : -1;
+        if (i < nrays) total += (unsigned long long)steps[i];
+        for (int k = 0; k < 6; k++) {
+            const unsigned m = __ballot_sync(kFull, st == k);
+            if (m && (threadIdx.x & 31) == 0) atomicAdd(sh + k, (unsigned long long)__popc(m));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(kFull, total, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(sh + 6, total);
+    __syncthreads();
+    if (threadIdx.x < 7 && sh[threadIdx.x]) atomicAdd(counts + threadIdx.x, sh[threadIdx.x]);
+}
+
 // Values of the run-length entries: the reference accumulates rayStep once per step by
 // repeated FP32 addition, starting from rayStep; the first (smallest) cell gets one extra
 // step and the source cell gets the final distance to the source (:243-276).
@@ -439,6 +462,14 @@ cudaError_t ray_sort(const RayLaunch &p, cudaStream_t st)
     long long g = (nrays + kSortWarps - 1) / kSortWarps;
     if (g > 148LL * 16) g = 148LL * 16;
     k_ray_sort<<<(int)(g > 0 ? g : 1), 32 * kSortWarps, 0, st>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t ray_stats(const int *status, const int *steps, int nrays, unsigned long long *counts, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemsetAsync(counts, 0, kRayCounts * sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    k_ray_stats<<<grid_for(nrays, 256), 256, 0, st>>>(status, steps, nrays, counts);
     return cudaGetLastError();
 }
 
