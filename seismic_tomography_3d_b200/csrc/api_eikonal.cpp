@@ -618,6 +618,18 @@ long long use_cluster(const tomo_ctx *ctx, const Batch &bt, const SolveCfg &c)
     return most <= ctx->cluster_bricks ? most : 0;
 }
 
+// Unbanded batches of many bricks run two bricks per warp at 8 warps x 3 CTAs per SM, when nothing
+// of the launch is asked for.  ms per call, two bricks | one: 64 shots of 201 x 201 x 101, windows
+// 5.63 | 5.80 (off the brick grid 5.94 | 6.17), whole 9.21 | 10.14; 16 shots (1.06 M bricks) 3.22 | 3.29;
+// 64 of 101 x 101 x 51 (0.56 M) 1.62 | 1.62; 4 of 201 x 201 x 101 (0.27 M) 1.43 | 1.33.
+void choose_pair(const Batch &bt, SolveCfg &c)
+{
+    if (!c.plain || c.time_band > 0.f || bt.q_total < (1ull << 20)) return;
+    c.pair = true;
+    c.block_warps = kBandBlockWarps;
+    c.occupancy = kBandOccupancy;
+}
+
 // Device buffers of a batch; uploads the descriptors and receiver positions.
 int upload_batch(tomo_ctx *ctx, const Batch &bt, int nrec, const tomo_point *receivers)
 {
@@ -806,6 +818,7 @@ int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_wind
     int rc = make_batch(ctx, nshots, shots, windows, nrec, receivers, bt);
     if (rc != TOMO_OK) return rc;
     cfg.cluster = use_cluster(ctx, bt, cfg);
+    choose_pair(bt, cfg);
     rc = upload_batch(ctx, bt, nrec, receivers);
     if (rc != TOMO_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream));  // host staging of upload_batch
@@ -864,6 +877,7 @@ int tomo_eik_solve(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tom
     int rc = make_batch(ctx, nshots, shots, windows, nrec, receivers, bt);
     if (rc != TOMO_OK) return rc;
     cfg.cluster = use_cluster(ctx, bt, cfg);
+    choose_pair(bt, cfg);
     ctx->have_solve = false;  // the pool is about to be overwritten
     rc = upload_batch(ctx, bt, nrec, receivers);
     if (rc != TOMO_OK) return rc;
