@@ -360,6 +360,13 @@ int tomo_ctx_destroy(tomo_ctx *ctx)
     ctx->fsm_T.release();
     ctx->fsm_shots.release();
     ctx->fsm_bar.release();
+    ctx->fsm_tab.release();
+    ctx->fsm_flags.release();
+    ctx->fim_keys.release();
+    ctx->band_min.release();
+    ctx->band_park.release();
+    ctx->band_pcnt.release();
+    ctx->tune_word.release();
     ctx->rec.release();
     ctx->t_recv.release();
     for (auto &ev : ctx->ev)
