@@ -435,9 +435,23 @@ estimated_models_folder = {d}/models/
                       "(the reference's count), FSM forward model, serial"}
 
 
+NO_REF = "the reference's sources are not here and its solvers are not built (oracle/_ref)"
+
+
+def have_reference():
+    import oracle
+
+    if not oracle.have_ref() and oracle.reference_src():
+        oracle.build()
+    return oracle.have_ref()
+
+
 def run_reference(args):
     rank, world, _ = rank_info()
     if rank != 0:
+        return 0
+    if not have_reference():
+        print(json.dumps({"impl": "reference", "unavailable": NO_REF}), flush=True)
         return 0
     sv = workload(0)
     per_step = []
@@ -646,12 +660,15 @@ def run_ours(args):
             line["inversion"] = inversion_object(args, iterations=3)
     # ---- CPU leg: the reference on the host cores, and the oracle as the checker ----------
     if cpu_leg:
-        rate, cores, desc = cpu_reference_sample(sv, max_shots=min(ns, max(8, 2 * (os.cpu_count() or 1))),
-                                                 budget_s=25.0)
-        line["cpu_baseline"] = {"value": rate, "unit": UNIT, "cores": cores, "kind": "reference", "sample": desc}
+        ref = have_reference()
+        line["cpu_baseline"] = {"unavailable": NO_REF}
+        if ref:
+            rate, cores, desc = cpu_reference_sample(sv, max_shots=min(ns, max(8, 2 * (os.cpu_count() or 1))),
+                                                     budget_s=25.0)
+            line["cpu_baseline"] = {"value": rate, "unit": UNIT, "cores": cores, "kind": "reference", "sample": desc}
         line["accuracy"] = oracle_accuracy(sv, acc_idx, acc_vols)
         if not args.headline_only:
-            line["config1"]["cpu"] = config1_cpu()
+            line["config1"]["cpu"] = config1_cpu() if ref else {"unavailable": NO_REF}
             line["tomography"]["reference_tomography_exe"] = reference_tomography_exe()
     if rank == 0:
         print(json.dumps(line), flush=True)
