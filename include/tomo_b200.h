@@ -86,7 +86,8 @@ typedef struct {
                         (s).  <= 0: exact (default)                                  */
     int ieee_sqrt;   /* 1: IEEE sqrtf in the local update; 0 (default): sqrt.approx  */
     int sweep_groups;/* TOMO_OP_NGB schedule.  0 (default): tile wavefront -- one warp
-                        per 16x8x8 tile of a sweep in shared memory, tiles in diagonal
+                        (eight where the tiles in flight are few, as for one shot) per
+                        16x8x8 tile of a sweep in shared memory, tiles in diagonal
                         order behind their upwind tiles, one grid barrier per sweep;
                         batches with a source on the last node of its window along an
                         axis take the plane schedule.  > 0: the diagonal-plane schedule
@@ -94,7 +95,7 @@ typedef struct {
                         sweeping their own shots.  Both are bit-exact with the reference
                         where every source lies off the far faces of its window.        */
     int schedule;    /* TOMO_OP_JW work schedule: TOMO_SCHED_DEFAULT, TOMO_SCHED_ROUNDS,
-                        TOMO_SCHED_ASYNC                                              */
+                        TOMO_SCHED_ASYNC, TOMO_SCHED_PAIR                             */
     float time_band; /* ROUNDS schedule, time-band ordering (s).  Every push carries the
                         smallest new time of the pushing brick; a queued brick whose key
                         is more than time_band above the smallest key its shot met in
@@ -132,8 +133,10 @@ typedef struct {
 #define TOMO_SCHED_ASYNC   2
 /* PAIR: the ROUNDS schedule with two 4x4x4 bricks per warp (16 lanes each, a y-column of 4
  *   nodes per lane), sharing the item fetch and queueing.  DEFAULT runs it for banded
- *   solves (time_band > 0) and when the autotuner chose it; ROUNDS keeps one brick per
- *   warp. */
+ *   solves (time_band > 0), when the autotuner chose it, and for batches of 2^20 bricks or
+ *   more whose launch shape is left to the library; ROUNDS keeps one brick per warp.
+ * DEFAULT also gives one thread-block cluster to each of up to four shots that fit a
+ *   cluster's shared memory, again with the launch shape left to the library. */
 #define TOMO_SCHED_PAIR    3
 
 typedef struct {
