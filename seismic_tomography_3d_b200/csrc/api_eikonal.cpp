@@ -226,7 +226,7 @@ int launch_ngb(tomo_ctx *ctx, const std::vector<ShotDesc> &sd, const tomo_point 
         p.flags = ctx->fsm_flags.ptr;
         p.cursors = ctx->fsm_bar.ptr + 2;
         p.shot_done = ctx->fsm_bar.ptr + 2 * ngroups + 16;
-        p.nan = p.shot_done + 16 * (size_t)nshots;
+        p.plain = p.shot_done + 16 * (size_t)nshots;
         p.shot_tiles = reinterpret_cast<const unsigned *>(ctx->fsm_tab.ptr + tab.size());
         p.widest = (int)widest;
     }

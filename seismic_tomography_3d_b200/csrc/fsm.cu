@@ -331,7 +331,8 @@ cudaError_t fsm_solve(const FsmLaunch &p, int *grid_out, cudaStream_t st)
 // arithmetic (lesser, by_sum, root) and the mirrored tile, whose plane loop has one form and no
 // index arithmetic for all eight octants, count: 64 shots of 201 x 201 x 101, windows of 60-100 %,
 // 48.6 -> 46.2 ms with the short division and no branches, 40.5 with the short root and the
-// mirrored tile, 38.5 with the one-instruction minimum (37.2 in the run that compared the whole call).
+// mirrored tile, 38.5 with the one-instruction minimum (36.9 for the whole call in a later run, and
+// 37.7 with std::min's order kept for NaN candidates, std_min).
 // -------------------------------------------------------------------------------------
 namespace {
 
@@ -352,10 +353,12 @@ static_assert(kFsmTZ >= kFsmTX && kFsmTZ >= kFsmTY && kMaxPlane <= 64, "a plane 
 
 // Arithmetic of the operator.  kFast: the short division and square root of common.cuh, the
 // same IEEE results in 3 and 6 instructions, and the hardware's minimum, one instruction where
-// std::min's order of comparison takes two.  The minimum differs for NaN only, and the short
-// forms turn an infinite candidate (zero velocity) into NaN, which that minimum drops as std::min
-// drops infinity.  So kFast is right as long as no slowness and no seed is NaN (the flag set
-// before the sweeps, FsmLaunch::nan) and the spacings suit the divisors; else the plain forms.
+// std::min's order of comparison takes two.  The minimum differs for NaN only.  A 2D candidate
+// is NaN where its discriminant is negative although its test holds (a diagonal neighbour that
+// no sweep has reached yet, at 1e6), and what std::min then drops is kept track of (std_min).
+// An infinite slowness or seed would make candidates infinite, which the short forms turn into
+// NaN; those and NaN itself are flagged before the sweeps (FsmLaunch::plain), and the model
+// takes the plain forms, as it does where the spacings do not suit the divisors.
 template <bool kFast>
 __device__ __forceinline__ float by_sum(float a, const Divisor &d)
 {
@@ -374,6 +377,16 @@ __device__ __forceinline__ float lesser(float a, float b)
     return kFast ? fminf(a, b) : smin(a, b);
 }
 
+// std::min(a, b) of candidates that may be NaN: NaN if a is, a if b is.
+template <bool kFast>
+__device__ __forceinline__ float std_min(float a, float b)
+{
+    if (!kFast) return smin(a, b);
+    float m;  // two instructions; fminf drops b's NaN
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(fminf(b, __int_as_float(0x7f800000))));
+    return m;
+}
+
 // The candidates of Accurate_FSM::inner_sweep (accurate_FSM.cpp:159-265) for the node at T, in
 // the reference's operation order (this file is compiled with -fmad=false).  The tile lies in
 // shared memory in the sweep's own direction on every axis (staging mirrors the axes it runs
@@ -382,7 +395,7 @@ __device__ __forceinline__ float lesser(float a, float b)
 // the operator's max(i - 1, 1) and min(i, n - 1) read the values at i - 1 and i: every minimum
 // comes from the node's 2 x 2 x 2 cell cube (halo indices i-1..i, j-1..j, k-1..k), mirrored
 // with the tile, so that its cell 0 on an axis is the upwind one (the reference's i1, j1, k1).
-// A minimum of numbers is exact and independent of its order, so each has the reference's value;
+// A minimum of slownesses is exact and independent of its order, so each has the reference's value;
 // with NaN it is not, and the plain form (not kFast) takes the cells in the reference's order,
 // lower index first on each axis (flip: bit 0 z, 1 x, 2 y, set where the tile is mirrored).
 constexpr int kDZ = 1, kDX = kPZ, kDY = kPZ * kPX;  // one step along each axis
@@ -411,8 +424,7 @@ __device__ __forceinline__ float candidate_2d(float a, float b, float da, float 
 }
 
 // Candidates of warp C: C = 0 z with (z, x), 1 y with (z, y), 2 x with (x, y), 3 the 3D one.
-// Every candidate is computed and kept only where the reference's test holds (a NaN from a
-// negative discriminant is dropped with it).  Skipping those no lane needs by a branch was
+// Every candidate is computed and kept only where the reference's test holds.  Skipping those no lane needs by a branch was
 // faster with the plain divisions and roots (48.6 vs 52.3 ms per 64-shot batch); with the short
 // division it costs more than it saves (48.5 vs 46.2 ms).
 template <int C, bool kFast>
@@ -507,9 +519,9 @@ template <bool kFast>
 __device__ __forceinline__ float least(const float *T, float z1, float x1, float y1, float zx, float zy, float xy,
                                        float zxy)
 {
-    const float t1D = lesser<kFast>(z1, lesser<kFast>(x1, y1)), t2D = lesser<kFast>(zx, lesser<kFast>(zy, xy));
+    const float t1D = lesser<kFast>(z1, lesser<kFast>(x1, y1)), t2D = std_min<kFast>(zx, std_min<kFast>(zy, xy));
     const bool above = lesser<kFast>(t1D, t2D) > smax(T[-kDZ], smax(T[-kDX], T[-kDY]));
-    return lesser<kFast>(T[0], lesser<kFast>(t1D, lesser<kFast>(t2D, above ? zxy : 1e6f)));
+    return lesser<kFast>(T[0], lesser<kFast>(t1D, std_min<kFast>(t2D, above ? zxy : 1e6f)));
 }
 
 // One tile, diagonal plane by diagonal plane, by one warp: all candidates of a node in its lane.
@@ -749,8 +761,8 @@ __global__ void __launch_bounds__(fsm_threads(kWarps), kWarps == 1 ? 2 : 1) k_fs
     if (kFast) {
         bool any = false;
         const long long n = (long long)p.nx * p.ny * p.nz;
-        for (long long q = gthread; q < n; q += nthreads) any |= isnan(__ldg(p.slow + q));
-        if (__any_sync(kFull, any) && lane == 0) atomicOr(p.nan, 1u);
+        for (long long q = gthread; q < n; q += nthreads) any |= !isfinite(__ldg(p.slow + q));
+        if (__any_sync(kFull, any) && lane == 0) atomicOr(p.plain, 1u);
     }
     if (!group_barrier(p.bar, gridDim.x, p.err, p.spin_limit)) return;
     for (long long q = gthread; q < (long long)p.nshots * 27; q += nthreads) {
@@ -761,11 +773,11 @@ __global__ void __launch_bounds__(fsm_threads(kWarps), kWarps == 1 ? 2 : 1) k_fs
         ShotGrid g{&s, p.T + s.t_off, 0, nxx, s.wny + 2, nzz};
         const float S0 = sget(p, g, s.sidz, s.sidx, s.sidy);
         const float t = S0 * s.seed_dist[e];
-        if (kFast && isnan(t)) atomicOr(p.nan, 1u);
+        if (kFast && !isfinite(t)) atomicOr(p.plain, 1u);
         __stcg(p.T + s.t_off + sid + oz + (long long)ox * nzz + (long long)oy * nxx * nzz, t);
     }
     if (!group_barrier(p.bar, gridDim.x, p.err, p.spin_limit)) return;
-    const bool nan = kFast && ld_volatile(p.nan) != 0u;
+    const bool plain = !kFast || ld_volatile(p.plain) != 0u;
 
     for (int q = 0; q < 16; q++) {
         const int sgz = fsm_sign_z(q), sgx = fsm_sign_x(q), sgy = fsm_sign_y(q);
@@ -862,7 +874,7 @@ __global__ void __launch_bounds__(fsm_threads(kWarps), kWarps == 1 ? 2 : 1) k_fs
             t.nb = nb;
             t.flip = (rz.di < 0 ? 1 : 0) | (rx.di < 0 ? 2 : 0) | (ry.di < 0 ? 4 : 0);
             t.full = t.nc >= kFsmTZ && t.na >= kFsmTX && t.nb >= kFsmTY;
-            if (kFast && !nan)
+            if (kFast && !plain)
                 relax_tile<kWarps, kFast>(p, t, lane, warp, group);
             else
                 relax_tile<kWarps, false>(p, t, lane, warp, group);
