@@ -133,7 +133,8 @@ __device__ __forceinline__ float fdiv(float a, const Divisor &d)
 // Square root: the hardware's reciprocal root r gives g = a r and h = r / 2, and one step with
 // the exact residual a - g g corrects g (Markstein 1990): five operations, the IEEE root for
 // every a in [2^-102, 2^126) (tests/test_sqrt_gpu.py goes through all of them) and NaN below
-// zero.  Below 2^-102 it can be an ulp off, and a = 0 is set apart.
+// zero.  Below 2^-102 it can be an ulp off, for subnormal a (whose reciprocal root is flushed to
+// infinity) and infinite a it is NaN, and a = 0 is set apart.  Callers keep a in the range.
 __device__ __forceinline__ float fsqrt(float a)
 {
     float r;

@@ -12,6 +12,9 @@
 // blocks form `ngroups` independent groups (shots g, g+ngroups, ...), each with its own
 // bounded barrier between planes.  The default schedule (k_fsm_tiled, below) orders the
 // same updates tile by tile instead of plane by plane.
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 #include "fsm.cuh"
 
@@ -357,8 +360,9 @@ static_assert(kFsmTZ >= kFsmTX && kFsmTZ >= kFsmTY && kMaxPlane <= 64, "a plane 
 // is NaN where its discriminant is negative although its test holds (a diagonal neighbour that
 // no sweep has reached yet, at 1e6), and what std::min then drops is kept track of (std_min).
 // An infinite slowness or seed would make candidates infinite, which the short forms turn into
-// NaN; those and NaN itself are flagged before the sweeps (FsmLaunch::plain), and the model
-// takes the plain forms, as it does where the spacings do not suit the divisors.
+// NaN, and a very small slowness takes the root's argument out of its range (fsm_solve_tiled);
+// those and NaN itself are flagged before the sweeps (FsmLaunch::plain), and the model takes the
+// plain forms, as it does where the spacings do not suit the divisors.
 template <bool kFast>
 __device__ __forceinline__ float by_sum(float a, const Divisor &d)
 {
@@ -761,7 +765,10 @@ __global__ void __launch_bounds__(fsm_threads(kWarps), kWarps == 1 ? 2 : 1) k_fs
     if (kFast) {
         bool any = false;
         const long long n = (long long)p.nx * p.ny * p.nz;
-        for (long long q = gthread; q < n; q += nthreads) any |= !isfinite(__ldg(p.slow + q));
+        for (long long q = gthread; q < n; q += nthreads) {
+            const float s = fabsf(__ldg(p.slow + q));
+            any |= !(s == 0.0f || (s >= p.s_lo && s <= p.s_hi));
+        }
         if (__any_sync(kFull, any) && lane == 0) atomicOr(p.plain, 1u);
     }
     if (!group_barrier(p.bar, gridDim.x, p.err, p.spin_limit)) return;
@@ -954,6 +961,12 @@ cudaError_t fsm_solve_tiled(const FsmLaunch &p, int *grid_out, cudaStream_t st)
     if (grid_out) *grid_out = grid;
     FsmLaunch pp = p;
     pp.sweep_barrier = split ? 1 : 0;
+    // Slownesses whose root arguments lie in fsqrt's range: the arguments are differences of
+    // 4 s^2 w (w: a sum of two inverse squared spacings) or 9 s^2 dsum and what is at most that, so
+    // they are 0 or at least 2^-25 of it, and below 2^126 as it is.  (Zero leaves no root but 0.)
+    const double wmin = std::min(std::min(p.by_zx.y, p.by_zy.y), p.by_xy.y);
+    pp.s_lo = (float)std::sqrt(0x1p-78 / wmin);
+    pp.s_hi = (float)std::min(0x1p60, std::sqrt(0x1p121 / (double)p.by_sum.y));
     void *args[] = {&pp};
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, st);
 }

@@ -95,7 +95,9 @@ struct FsmLaunch {
     int tab_base[16], tab_nd[16];
     unsigned *flags;          // per tile: last sweep (q + 1) that finished it
     unsigned *cursors;        // 16 tile cursors, zeroed before the launch
-    unsigned *plain;          // set if a slowness or a seeded time is not finite (zeroed before the launch)
+    unsigned *plain;          // set if a slowness or a seeded time does not suit the short arithmetic
+                              // (zeroed before the launch)
+    float s_lo, s_hi;         // slownesses that do: 0 and these (set by fsm_solve_tiled)
     unsigned *shot_done;      // per shot and sweep: tiles finished (16 x nshots, zeroed)
     const unsigned *shot_tiles;  // per shot and sweep: tiles of the sweep (16 x nshots)
     int widest;               // most tiles of all shots on one diagonal of a full sweep

@@ -37,3 +37,11 @@ def test_scattered_slow_nodes(tomo, velocity, seed):
     node = (rng.integers(1, nx - 3), rng.integers(1, ny - 3), rng.integers(0, nz - 3))
     with np.errstate(divide="ignore"):
         _both(tomo, np.float32(1.0) / v, 25.0, node, 240)
+
+
+@pytest.mark.parametrize("exponent", [-64, -60, -54, -36, -35, -34, 30], ids=str)
+def test_tiny_slowness(tomo, exponent):
+    """Root arguments of about 2^(2 exponent - 7); at this spacing the short forms take slownesses from
+    2^-34.9 up."""
+    slow = (np.random.default_rng(abs(exponent)).uniform(1.0, 2.0, (44, 60, 30)) * 2.0 ** exponent).astype(np.float32)
+    _both(tomo, slow, 25.0, (7, 30, 0), 90)
