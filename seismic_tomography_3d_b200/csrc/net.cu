@@ -538,7 +538,9 @@ __device__ __forceinline__ void axis_weight(int x, int k, int n, int &c0, int &c
 // division and runs of 32), 83 % of the issue slots.
 constexpr int kTimeRun = 64;
 
-template <bool kStrided>
+// kFast: the short root of common.cuh; else the IEEE root.  Squared distances of spacings in
+// [2^-50, 2^30] lie in the short root's range, or below h^2, where the time is 0 either way.
+template <bool kStrided, bool kFast>
 __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, const float *tau, float *t_out)
 {
     const Job j = jobs[blockIdx.z];
@@ -593,7 +595,7 @@ __global__ void __launch_bounds__(256) k_tau_to_time(const Job *jobs, float h, c
                 }
             }
             const float ex = x * h - j.sx;
-            const float dist = fsqrt(ex * ex + ey * ey + ez * ez);
+            const float d2 = ex * ex + ey * ey + ez * ez, dist = kFast ? fsqrt(d2) : sqrtf(d2);
             float t = 0.f;
             if (dist >= h) {
                 if (kStrided) {
@@ -753,10 +755,10 @@ cudaError_t tau_to_time(const Job *jobs, int njobs, float h, int stride, const f
     if (njobs < 1 || njobs > 65535 || max_plane < 1 || max_wnx < 1) return cudaErrorInvalidValue;
     const int runs = (max_wnx + kTimeRun - 1) / kTimeRun;
     const dim3 grid((unsigned)((max_plane + 255) / 256), (unsigned)(runs < 65535 ? runs : 65535), (unsigned)njobs);
-    if (stride > 1)
-        k_tau_to_time<true><<<grid, 256, 0, st>>>(jobs, h, tau, t_out);
-    else
-        k_tau_to_time<false><<<grid, 256, 0, st>>>(jobs, h, tau, t_out);
+    const bool fast = h >= 0x1p-50f && h <= 0x1p30f;
+    auto fn = stride > 1 ? (fast ? k_tau_to_time<true, true> : k_tau_to_time<true, false>)
+                         : (fast ? k_tau_to_time<false, true> : k_tau_to_time<false, false>);
+    fn<<<grid, 256, 0, st>>>(jobs, h, tau, t_out);
     return cudaGetLastError();
 }
 
