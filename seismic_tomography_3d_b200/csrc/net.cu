@@ -419,8 +419,9 @@ __global__ void __launch_bounds__(256) k_head_bwd(const bf16 *y, const float *wh
         float f[16], d0[8], d1[8];
         load16(y, v, f);
         s[16] += g;
+        if (g != 0.f)  // an infinite activation where there is no loss adds nothing, not 0 x inf
 #pragma unroll
-        for (int k = 0; k < 16; k++) s[k] += g * f[k];
+            for (int k = 0; k < 16; k++) s[k] += g * f[k];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             d0[k] = f[k] > 0.f ? g * w[k] : 0.f;
