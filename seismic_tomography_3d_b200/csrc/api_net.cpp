@@ -487,9 +487,10 @@ int tomo_net_predict_strided(tomo_net *net, int n, const tomo_net_sample *sample
         NK(tomo::net::features(net->jobs.ptr, cnt, h, net->act[X].ptr, per, net->stream));
         rc = forward(net, v, false);
         if (rc != TOMO_OK) return rc;
-        int max_plane = 1, max_wnx = 1;
+        long long max_plane = 1;
+        int max_wnx = 1;
         for (const auto &j : jobs) {
-            max_plane = std::max(max_plane, j.nz * j.wny);
+            max_plane = std::max(max_plane, (long long)j.nz * j.wny);
             max_wnx = std::max(max_wnx, j.wnx);
         }
         NK(tomo::net::tau_to_time(net->jobs.ptr, cnt, h, stride, net->tau.ptr, t_pred + nat, max_plane, max_wnx,

@@ -86,7 +86,7 @@ cudaError_t tau_target(const Job *jobs, int njobs, float h, float *tau, long lon
 // distance < h: no ceiling there); jobs with stride > 1 interpolate tau trilinearly between
 // the sampled nodes first (max_plane, max_wnx: the largest nz * wny and wnx of the jobs)
 cudaError_t tau_to_time(const Job *jobs, int njobs, float h, int stride, const float *tau, float *t_out,
-                        int max_plane, int max_wnx, cudaStream_t st);
+                        long long max_plane, int max_wnx, cudaStream_t st);
 
 // Seeded random layered models (training data): one 64^3-like tile per entry of `tiles`,
 // written as slowness into the natural-layout model of size nz x nx x ny.

@@ -6,6 +6,8 @@ also where squared distances leave the short root's range.
 
 A sample without a single target (all its traveltimes 0) takes no part in the loss: the head's
 gradient is the other sample's alone, also where the untargeted sample's activations overflow.
+
+A window whose vertical section has more than 2^31 nodes is predicted in full.
 """
 import numpy as np
 import pytest
@@ -76,3 +78,23 @@ def test_untargeted_sample_leaves_the_head_alone(tomo):
     assert np.isfinite(g1[head:]).all() and g1[head] != 0
     # the same sums in other groups: a few hundred terms, 6e-8 each
     np.testing.assert_allclose(g2[head:], g1[head:], rtol=1e-5, atol=0)
+
+
+def test_more_than_2_31_nodes_in_a_section(tomo):
+    import torch
+
+    nx, ny, nz, h = 2, 46341, 46342, 10.0
+    if torch.cuda.mem_get_info()[0] < 110e9:
+        pytest.skip("needs 110 GB of device memory")
+    slow = torch.full((ny, nx, nz), 4e-4, dtype=torch.float32, device="cuda")
+    out = torch.full((ny, nx, nz), -7.0, dtype=torch.float32, device="cuda")
+    net = tomo.Net(seed=2)
+    net.predict([dict(slow=slow.data_ptr(), model_nx=nx, model_ny=ny, nz=nz, window=(0, nx, 0, ny), T=0,
+                      source=(0.0, 0.0, 0.0))], h, out.data_ptr(), stride=16)
+    net.close()
+    missing = sum(int((out[k:k + 4096] == -7.0).sum()) for k in range(0, ny, 4096))
+    corner = [float(out[y, 0, z]) / (4e-4 * h * (y * y + z * z) ** 0.5) for y, z in ((ny - 1, nz - 1), (ny - 1, 0), (0, nz - 1))]
+    del slow, out
+    torch.cuda.empty_cache()
+    assert missing == 0
+    assert np.isfinite(corner).all() and 0.0 not in corner
