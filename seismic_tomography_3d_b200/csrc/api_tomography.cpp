@@ -203,6 +203,7 @@ int jac_prepare(tomo_ctx *ctx, const tomo_jacobian_opts *opts, JacGeom &jg)
     jg.dz = opts->dz;
     bool full = true;
     for (const auto &d : ctx->shots_h) full = full && d.wx0 == 0 && d.wy0 == 0 && d.wnx == g.nx && d.wny == g.ny;
+    jg.wide = wide_fields(ctx->shots_h.data(), ctx->shots_h.size());
     if (jg.illum && !full) return fail(ctx, TOMO_ERR_INVALID_ARG, "illumination needs full-model windows");
 
     const long long nrays = jg.nrays;
@@ -255,8 +256,7 @@ RayLaunch ray_launch(tomo_ctx *ctx, const JacGeom &jg)
     const tomo_grid &g = ctx->g;
     RayLaunch rl{};
     rl.T = ctx->T.ptr;
-    for (const auto &d : ctx->shots_h)
-        rl.wide = rl.wide || (long long)d.nbx * d.nby * d.nbz * kBrickNodes >= (1ll << 31);
+    rl.wide = jg.wide;
     rl.shots = ctx->shots_d.ptr;
     rl.nshots = ctx->nshots;
     rl.spos = ctx->spos.ptr;

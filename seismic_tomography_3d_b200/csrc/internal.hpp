@@ -15,6 +15,7 @@ struct JacGeom {
     long long M, N, nrays, tk_entries;
     int max_steps, cap_runs;
     bool ray_cap, illum;
+    bool wide;  // some field has 2^31 nodes or more (chooses the march's kernel, so a graph's key holds it)
     float rayStep, dx, dy, dz;
 };
 

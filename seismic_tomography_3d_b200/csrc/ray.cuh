@@ -19,10 +19,18 @@ enum RayStatus : int {
     kRayOverflow = 5,  // more distinct cells than the per-ray capacity
 };
 
+// Whether the march needs 64-bit offsets: some field has 2^31 nodes or more.
+inline bool wide_fields(const ShotDesc *shots, size_t n)
+{
+    for (size_t i = 0; i < n; i++)
+        if ((long long)shots[i].nbx * shots[i].nby * shots[i].nbz * kBrickNodes >= (1ll << 31)) return true;
+    return false;
+}
+
 struct RayLaunch {
     const int *order;     // rays in march order (nullptr: natural order)
     const float *T;
-    int wide;             // some field has 2^31 nodes or more (64-bit offsets)
+    int wide;             // wide_fields: 64-bit offsets
     const ShotDesc *shots;
     int nshots;
     const float *spos;    // 3*nshots: x | y | z (metres)
