@@ -202,6 +202,17 @@ int tomo_eik_solve(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tom
                    int nrec, const tomo_point *receivers, float *t_recv,
                    const tomo_eik_opts *opts, tomo_eik_stats *stats);
 
+/* Kernel that the last solve of the context ran (tomo_eik_solve, _solve_seeded, _autotune's last
+ * trial or tomo_iteration). */
+#define TOMO_KERNEL_NONE    0  /* no solve yet                                                   */
+#define TOMO_KERNEL_SOLVE   1  /* rounds, one 4x4x4 brick per warp                               */
+#define TOMO_KERNEL_PAIR    2  /* rounds, two 4x4x4 bricks per warp                              */
+#define TOMO_KERNEL_CLUSTER 3  /* one thread-block cluster per shot, its field in shared memory  */
+#define TOMO_KERNEL_BRICK8  4  /* rounds, 8x8x8 bricks                                           */
+#define TOMO_KERNEL_ASYNC   5  /* asynchronous schedule                                          */
+#define TOMO_KERNEL_SWEEPS  6  /* TOMO_OP_NGB                                                    */
+int tomo_eik_kernel(const tomo_ctx *ctx);
+
 /* Copies the traveltime field of shot `shot` of the last solve to the host, cropped to
  * its window: wz*wx*wy floats (z fastest) -- Eikonal::travel_time after
  * eikonal_equation (block_FIM.cpp:59-69, 371-401). */

@@ -26,6 +26,9 @@ ERRORS = {
     -9: "TOMO_ERR_CAPACITY",
 }
 
+# tomo_eik_kernel: TOMO_KERNEL_* -> the kernel's name
+KERNELS = (None, "k_fim_solve", "k_fim_pair", "k_fim_cluster", "k_fim_solve8", "k_fim_async", "k_fsm")
+
 
 class TomoError(RuntimeError):
     def __init__(self, status, msg):
@@ -111,6 +114,7 @@ def load_library(path: str = LIB_PATH):
     lib.tomo_eik_window.argtypes = [V, I, P(Window)]
     lib.tomo_eik_brick_shapes.argtypes = [P(I), I]
     lib.tomo_eik_volumes.argtypes = [V, V]
+    lib.tomo_eik_kernel.argtypes = [V]
     lib.tomo_eik_autotune.argtypes = [V, I, P(Point), P(Window), I, P(EikOpts), P(TuneStats)]
     lib.tomo_eik_solve_seeded.argtypes = [V, I, P(Point), P(Window), I, P(Point), V, V, F, P(EikOpts),
                                           P(EikStats), P(SeedStats)]
@@ -380,6 +384,10 @@ class Context:
         shape = {"brick": best.brick, "block_warps": best.block_warps, "occupancy": best.occupancy,
                  "max_inner": best.max_inner, "time_band": best.time_band, "schedule": best.schedule}
         return shape, {f: getattr(st, f) for f, _ in st._fields_}
+
+    def eik_kernel(self):
+        """Kernel of the last solve: one of KERNELS."""
+        return KERNELS[self.lib.tomo_eik_kernel(self.h)]
 
     def volume_sizes(self, nshots, windows=None):
         """Floats of each shot's window volume (nz*wx*wy) in the back-to-back layout."""

@@ -753,10 +753,18 @@ int enqueue_fim(tomo_ctx *ctx, const tomo::FimLaunch &p, size_t t_total, size_t 
     if (c.cluster > 0) {
         CK(tomo::fim_init(nullptr, 0, nullptr, 0, p.ctrl, p.stats, ctx->stream));
         if (ev_solve) CK(cudaEventRecord(ev_solve, ctx->stream));
-        if (tomo::fim_solve_cluster(p, c.cluster, c.ieee_sqrt, ctx->stream) == cudaSuccess) return TOMO_OK;
+        const cudaError_t e = tomo::fim_solve_cluster(p, c.cluster, ctx->cluster_bricks, c.ieee_sqrt, ctx->stream);
+        if (e == cudaSuccess) {
+            ctx->eik_kernel = TOMO_KERNEL_CLUSTER;
+            return TOMO_OK;
+        }
         (void)cudaGetLastError();
         ctx->cluster_bricks = 0;  // no place for a cluster: the grid-wide kernel, now and later
     }
+    ctx->eik_kernel = c.brick8 ? TOMO_KERNEL_BRICK8
+                      : c.async ? TOMO_KERNEL_ASYNC
+                      : p.pair  ? TOMO_KERNEL_PAIR
+                                : TOMO_KERNEL_SOLVE;
     if (c.brick8) {
         CK(tomo::fim_init(p.T, t_total, p.qflag, (size_t)p.list_cap, p.ctrl, p.stats, ctx->stream));
         CK(tomo::fim_seed8(p.shots, p.nshots, p.S, p.gbx, p.gbz, p.T, p.qflag, p.lists, p.local_bits, p.ctrl,
@@ -895,6 +903,7 @@ int tomo_eik_solve(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tom
     if (opts && opts->op == TOMO_OP_NGB) {
         rc = launch_ngb(ctx, bt.sd, shots, nshots, nrec, opts->sweep_groups, cfg.spin_limit);
         if (rc != TOMO_OK) return rc;
+        ctx->eik_kernel = TOMO_KERNEL_SWEEPS;
     } else {
         const tomo::FimLaunch p = fim_params(ctx, bt, cfg, nrec);
         rc = enqueue_fim(ctx, p, (size_t)bt.t_total, (size_t)bt.q_total, cfg, ctx->ev[3]);
@@ -959,6 +968,7 @@ int tomo_eik_solve_seeded(tomo_ctx *ctx, int nshots, const tomo_point *shots, co
                       ctx->lists.ptr, bt.local_bits, ctx->ctrl.ptr, ctx->stream, cfg.async ? 3 * (size_t)bt.q_total : 0));
     CK(cudaEventRecord(ev[3], ctx->stream));
     tomo::FimLaunch p = fim_params(ctx, bt, cfg, 0);
+    ctx->eik_kernel = cfg.async ? TOMO_KERNEL_ASYNC : p.pair ? TOMO_KERNEL_PAIR : TOMO_KERNEL_SOLVE;
     int grid = 0;
     CK(tomo::fim_solve(p, cfg.block_warps, cfg.occupancy, cfg.ieee_sqrt, &grid, ctx->stream, cfg.async));
     CK(cudaEventRecord(ev[4], ctx->stream));
@@ -1263,6 +1273,8 @@ int tomo_eik_window(tomo_ctx *ctx, int shot, tomo_window *out)
     *out = tomo_window{d.wx0, d.wx0 + d.wnx, d.wy0, d.wy0 + d.wny};
     return TOMO_OK;
 }
+
+int tomo_eik_kernel(const tomo_ctx *ctx) { return ctx ? ctx->eik_kernel : TOMO_KERNEL_NONE; }
 
 int tomo_eik_volume(tomo_ctx *ctx, int shot, float *t_out)
 {

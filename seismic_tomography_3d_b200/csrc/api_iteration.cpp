@@ -192,11 +192,13 @@ extern "C" int tomo_iteration(tomo_ctx *ctx, int nshots, const tomo_point *shots
         G.key_a.clear();
         if (capture(ctx, &G.a, stage_a) == TOMO_OK) {
             G.key_a = key_a;
+            G.kernel = ctx->eik_kernel;
             captured = 1;
         }
     }
     if (graphs && G.a) {
         CK(cudaGraphLaunch(G.a, ctx->stream));
+        ctx->eik_kernel = G.kernel;
     } else {
         replayed = 0;
         if (graphs) G.broken = true;  // capture refused: eager from now on

@@ -43,6 +43,7 @@ struct IterGraphs {
     std::vector<char> key_a, key_b;  // options, sizes and device addresses baked in
     long long cap = 0;               // Jacobian capacity graph B was built for
     unsigned long long *pinned = nullptr;
+    int kernel = 0;                  // TOMO_KERNEL_* of the solve in graph A
     bool broken = false;             // capture refused once: run eagerly from then on
 };
 
@@ -97,6 +98,7 @@ struct tomo_ctx {
     bool have_solve = false;
     // launch shape chosen by tomo_eik_autotune (0: not tuned)
     int cluster_bricks = 0;       // largest shot one cluster can hold (fim_cluster_limit)
+    int eik_kernel = 0;           // TOMO_KERNEL_* of the last solve
     int tuned_block_warps = 0, tuned_occupancy = 0, tuned_max_inner = 0;
     int tuned_brick = 0;          // 0: none chosen (4^3); TOMO_BRICK_4 / TOMO_BRICK_8
     int tuned_schedule = 0;       // 0: none chosen (rounds); TOMO_SCHED_PAIR

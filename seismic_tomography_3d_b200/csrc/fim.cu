@@ -2259,9 +2259,11 @@ static cudaError_t launch_pair(const FimLaunch &p, int block_warps, int *grid_ou
                                       : (const void *)k_fim_pair<MINB, kFastSqrt, false>);
     const int threads = 32 * block_warps;
     // per warp: two tiles, the push buffer, and (time band) the pushes' keys and parked items
-    const size_t smem = (size_t)block_warps * (2 * kTileNodes * sizeof(float) + kPushCap * sizeof(unsigned) +
-                                               (band ? (kPushCap + kParkCap) * sizeof(unsigned) : 0));
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t per_warp = 2 * kTileNodes * sizeof(float) + kPushCap * sizeof(unsigned) +
+                            (band ? (kPushCap + kParkCap) * sizeof(unsigned) : 0);
+    const size_t smem = block_warps * per_warp;
+    // what 16 warps take: the limit is the kernel's, and another context may launch it meanwhile
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(16 * per_warp));
     if (e != cudaSuccess) return e;
     int dev = 0, nsm = 0, per_sm = 0;
     e = cudaGetDevice(&dev);
@@ -2355,11 +2357,15 @@ cudaError_t fim_cluster_limit(int *max_bricks)
     return cudaSuccess;
 }
 
-cudaError_t fim_solve_cluster(const FimLaunch &p, long long max_bricks, bool ieee_sqrt, cudaStream_t st)
+cudaError_t fim_solve_cluster(const FimLaunch &p, long long bricks, int max_bricks, bool ieee_sqrt, cudaStream_t st)
 {
-    const int cap = (int)((max_bricks + (int)kClusterCtas - 1) / (int)kClusterCtas);
+    if (bricks < 1 || bricks > max_bricks) return cudaErrorInvalidValue;
+    const int cap = (int)((bricks + (int)kClusterCtas - 1) / (int)kClusterCtas);
     const void *fn = cluster_kernel(ieee_sqrt, p.gather != 0);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cluster_smem(cap));
+    // what the largest shot takes: the limit is the kernel's, and another context may launch it
+    // meanwhile (set to this shot's need, it could be lowered between the set and the launch)
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)cluster_smem(max_bricks / (int)kClusterCtas));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr;

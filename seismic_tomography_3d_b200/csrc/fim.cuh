@@ -128,10 +128,10 @@ cudaError_t fim_solve(const FimLaunch &p, int block_warps, int occupancy, bool i
                       cudaStream_t st, bool async = false);
 // One shot per thread-block cluster, its field in shared memory (k_fim_cluster): for a few shots
 // of at most *max_bricks bricks each (what the current device's shared memory holds).  Needs
-// neither seed nor pool reset; p.ctrl and p.stats zeroed.  An error means that nothing was launched
-// (no place for a cluster of 16).
+// neither seed nor pool reset; p.ctrl and p.stats zeroed.  bricks: of the largest shot.  An error means
+// that nothing was launched (no place for a cluster of 16).
 cudaError_t fim_cluster_limit(int *max_bricks);
-cudaError_t fim_solve_cluster(const FimLaunch &p, long long max_bricks, bool ieee_sqrt, cudaStream_t st);
+cudaError_t fim_solve_cluster(const FimLaunch &p, long long bricks, int max_bricks, bool ieee_sqrt, cudaStream_t st);
 // 8^3 bricks, rounds schedule: work items are (shot, 8^3 group); p.qflag / p.list_cap are
 // the group queue flags and count; seeded by fim_seed8.  One CTA of 8 warps per group.
 cudaError_t fim_solve8(const FimLaunch &p, int occupancy, bool ieee_sqrt, int *grid_out, cudaStream_t st);
