@@ -758,8 +758,9 @@ int enqueue_fim(tomo_ctx *ctx, const tomo::FimLaunch &p, size_t t_total, size_t 
             ctx->eik_kernel = TOMO_KERNEL_CLUSTER;
             return TOMO_OK;
         }
+        if (!tomo::no_place_for_cluster(e)) CK(e);
         (void)cudaGetLastError();
-        ctx->cluster_bricks = 0;  // no place for a cluster: the grid-wide kernel, now and later
+        ctx->cluster_bricks = 0;  // the grid-wide kernel, now and later
     }
     ctx->eik_kernel = c.brick8 ? TOMO_KERNEL_BRICK8
                       : c.async ? TOMO_KERNEL_ASYNC

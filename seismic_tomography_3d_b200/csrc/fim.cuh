@@ -129,9 +129,15 @@ cudaError_t fim_solve(const FimLaunch &p, int block_warps, int occupancy, bool i
 // One shot per thread-block cluster, its field in shared memory (k_fim_cluster): for a few shots
 // of at most *max_bricks bricks each (what the current device's shared memory holds).  Needs
 // neither seed nor pool reset; p.ctrl and p.stats zeroed.  bricks: of the largest shot.  An error means
-// that nothing was launched (no place for a cluster of 16).
+// that nothing was launched; no_place_for_cluster: that the device cannot hold a cluster of 16 (the
+// grid-wide kernel can run instead), and not that something else is wrong.
 cudaError_t fim_cluster_limit(int *max_bricks);
 cudaError_t fim_solve_cluster(const FimLaunch &p, long long bricks, int max_bricks, bool ieee_sqrt, cudaStream_t st);
+inline bool no_place_for_cluster(cudaError_t e)
+{
+    return e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidConfiguration ||
+           e == cudaErrorNotSupported;
+}
 // 8^3 bricks, rounds schedule: work items are (shot, 8^3 group); p.qflag / p.list_cap are
 // the group queue flags and count; seeded by fim_seed8.  One CTA of 8 warps per group.
 cudaError_t fim_solve8(const FimLaunch &p, int occupancy, bool ieee_sqrt, int *grid_out, cudaStream_t st);
