@@ -475,6 +475,7 @@ struct SolveCfg {
     bool brick8;      // 8^3 bricks (one CTA per 2 x 2 x 2 group of storage bricks)
     bool plain;       // launch shape, schedule and wait limit all left to the library
     long long cluster;  // > 0: one cluster per shot, the largest of this many bricks (use_cluster)
+    int ctas;           // one-brick rounds kernel: CTAs per SM, 0: as many as fit (choose_grid)
 };
 
 SolveCfg solve_cfg(const tomo_ctx *ctx, const tomo_eik_opts *opts)
@@ -637,6 +638,14 @@ void choose_pair(const Batch &bt, SolveCfg &c)
     c.occupancy = kBandOccupancy;
 }
 
+// CTAs per SM of the one-brick rounds kernel.
+void choose_grid(const Batch &bt, SolveCfg &c)
+{
+    double fronts = 0.0;
+    for (const ShotDesc &d : bt.sd) fronts += std::pow((double)d.nbx * d.nby * d.nbz, 2.0 / 3.0);
+    c.ctas = tomo::rounds_ctas_per_sm(!c.plain || c.time_band > 0.f, bt.q_total, fronts);
+}
+
 // Device buffers of a batch; uploads the descriptors and receiver positions.
 int upload_batch(tomo_ctx *ctx, const Batch &bt, int nrec, const tomo_point *receivers)
 {
@@ -779,7 +788,7 @@ int enqueue_fim(tomo_ctx *ctx, const tomo::FimLaunch &p, size_t t_total, size_t 
                       ctx->stream, c.async ? 3 * (size_t)p.list_cap : 0));
     CK(band_reset(ctx, p));
     if (ev_solve) CK(cudaEventRecord(ev_solve, ctx->stream));
-    CK(tomo::fim_solve(p, c.block_warps, c.occupancy, c.ieee_sqrt, &grid, ctx->stream, c.async));
+    CK(tomo::fim_solve(p, c.block_warps, c.occupancy, c.ieee_sqrt, &grid, ctx->stream, c.async, c.ctas));
     return TOMO_OK;
 }
 
@@ -835,6 +844,7 @@ int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_wind
     if (rc != TOMO_OK) return rc;
     cfg.cluster = use_cluster(ctx, bt, cfg);
     choose_pair(bt, cfg);
+    choose_grid(bt, cfg);
     rc = upload_batch(ctx, bt, nrec, receivers);
     if (rc != TOMO_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream));  // host staging of upload_batch
@@ -848,6 +858,7 @@ int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_wind
     plan.async = cfg.async;
     plan.brick8 = cfg.brick8;
     plan.cluster = cfg.cluster;
+    plan.ctas = cfg.ctas;
     plan.t_total = (size_t)bt.t_total;
     plan.q_total = (size_t)bt.q_total;
     return TOMO_OK;
@@ -862,6 +873,7 @@ int eik_enqueue(tomo_ctx *ctx, const EikPlan &plan)
     c.async = plan.async;
     c.brick8 = plan.brick8;
     c.cluster = plan.cluster;
+    c.ctas = plan.ctas;
     return enqueue_fim(ctx, plan.p, plan.t_total, plan.q_total, c, nullptr);
 }
 
@@ -894,6 +906,7 @@ int tomo_eik_solve(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tom
     if (rc != TOMO_OK) return rc;
     cfg.cluster = use_cluster(ctx, bt, cfg);
     choose_pair(bt, cfg);
+    choose_grid(bt, cfg);
     ctx->have_solve = false;  // the pool is about to be overwritten
     rc = upload_batch(ctx, bt, nrec, receivers);
     if (rc != TOMO_OK) return rc;
@@ -954,6 +967,7 @@ int tomo_eik_solve_seeded(tomo_ctx *ctx, int nshots, const tomo_point *shots, co
     Batch bt;
     int rc = make_batch(ctx, nshots, shots, windows, nrec, receivers, bt);
     if (rc != TOMO_OK) return rc;
+    choose_grid(bt, cfg);
     ctx->have_solve = false;  // the pool is about to be overwritten
     rc = upload_batch(ctx, bt, nrec, receivers);
     if (rc != TOMO_OK) return rc;
@@ -971,7 +985,8 @@ int tomo_eik_solve_seeded(tomo_ctx *ctx, int nshots, const tomo_point *shots, co
     tomo::FimLaunch p = fim_params(ctx, bt, cfg, 0);
     ctx->eik_kernel = cfg.async ? TOMO_KERNEL_ASYNC : p.pair ? TOMO_KERNEL_PAIR : TOMO_KERNEL_SOLVE;
     int grid = 0;
-    CK(tomo::fim_solve(p, cfg.block_warps, cfg.occupancy, cfg.ieee_sqrt, &grid, ctx->stream, cfg.async));
+    CK(tomo::fim_solve(p, cfg.block_warps, cfg.occupancy, cfg.ieee_sqrt, &grid, ctx->stream, cfg.async,
+                       cfg.ctas));
     CK(cudaEventRecord(ev[4], ctx->stream));
     // 2. check: a node below what its neighbours give came from a ceiling below the truth
     CK(cudaMemsetAsync(ctx->viol.ptr, 0, (size_t)nshots * 3 * sizeof(unsigned long long), ctx->stream));
@@ -1014,7 +1029,8 @@ int tomo_eik_solve_seeded(tomo_ctx *ctx, int nshots, const tomo_point *shots, co
         tomo::FimLaunch p2 = p;
         p2.shots = ctx->shots_redo.ptr;
         p2.nshots = nredo;
-        CK(tomo::fim_solve(p2, cfg.block_warps, cfg.occupancy, cfg.ieee_sqrt, &grid, ctx->stream, cfg.async));
+        CK(tomo::fim_solve(p2, cfg.block_warps, cfg.occupancy, cfg.ieee_sqrt, &grid, ctx->stream, cfg.async,
+                       cfg.ctas));
         rc = read_solve(ctx, rounds2, act2, inner2, cfg);
         if (rc != TOMO_OK) return rc;
     }

@@ -185,6 +185,7 @@ extern "C" int tomo_iteration(tomo_ctx *ctx, int nshots, const tomo_point *shots
         push(key_a, p);
     push(key_a, plan.brick8);
     push(key_a, plan.cluster);
+    push(key_a, plan.ctas);
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     if (graphs && (!G.a || key_a != G.key_a)) {
         if (G.a) cudaGraphExecDestroy(G.a);

@@ -2281,7 +2281,8 @@ static cudaError_t launch_pair(const FimLaunch &p, int block_warps, int *grid_ou
 }
 
 template <int MINB, bool kFastSqrt>
-static cudaError_t launch_solve(const FimLaunch &p, int block_warps, bool async, int *grid_out, cudaStream_t st)
+static cudaError_t launch_solve(const FimLaunch &p, int block_warps, bool async, int ctas_per_sm, int *grid_out,
+                                cudaStream_t st)
 {
     const bool band = !async && p.band > 0.f;
     if (!async && p.pair) return launch_pair<MINB, kFastSqrt>(p, block_warps, grid_out, st);
@@ -2303,12 +2304,7 @@ static cudaError_t launch_solve(const FimLaunch &p, int block_warps, bool async,
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    // Few bricks: one CTA per SM, since a round then lasts as long as its chain of accesses and its
-    // barrier, which half the CTAs reach sooner.  ms per call, one | two: 1 shot of 3,375 bricks 0.31 |
-    // 0.36, of 8,788 0.40 | 0.49, of 66,300 0.84 | 0.95, 2 of them 0.99 | 1.05; but 4 of them 1.39 | 1.33,
-    // 16 of 8,788 0.78 | 0.78.
-    const bool few = !async && block_warps >= 16 && p.list_cap <= 131072u;
-    const int grid = nsm * (few ? 1 : per_sm);
+    const int grid = nsm * (ctas_per_sm > 0 && ctas_per_sm < per_sm ? ctas_per_sm : per_sm);
     if (grid_out) *grid_out = grid;
     FimLaunch pp = p;
     void *args[] = {&pp};
@@ -2316,25 +2312,25 @@ static cudaError_t launch_solve(const FimLaunch &p, int block_warps, bool async,
 }
 
 template <bool kFastSqrt>
-static cudaError_t solve_occ(const FimLaunch &p, int block_warps, int occupancy, bool async, int *grid_out,
-                             cudaStream_t st)
+static cudaError_t solve_occ(const FimLaunch &p, int block_warps, int occupancy, bool async, int ctas_per_sm,
+                             int *grid_out, cudaStream_t st)
 {
     switch (occupancy) {
-    case 1: return launch_solve<1, kFastSqrt>(p, block_warps, async, grid_out, st);
-    case 2: return launch_solve<2, kFastSqrt>(p, block_warps, async, grid_out, st);
-    case 3: return launch_solve<3, kFastSqrt>(p, block_warps, async, grid_out, st);
-    case 5: return launch_solve<5, kFastSqrt>(p, block_warps, async, grid_out, st);
-    case 6: return launch_solve<6, kFastSqrt>(p, block_warps, async, grid_out, st);
-    default: return launch_solve<4, kFastSqrt>(p, block_warps, async, grid_out, st);
+    case 1: return launch_solve<1, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
+    case 2: return launch_solve<2, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
+    case 3: return launch_solve<3, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
+    case 5: return launch_solve<5, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
+    case 6: return launch_solve<6, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
+    default: return launch_solve<4, kFastSqrt>(p, block_warps, async, ctas_per_sm, grid_out, st);
     }
 }
 
 cudaError_t fim_solve(const FimLaunch &p, int block_warps, int occupancy, bool ieee_sqrt, int *grid_out,
-                      cudaStream_t st, bool async)
+                      cudaStream_t st, bool async, int ctas_per_sm)
 {
     if (block_warps < 1 || block_warps > 16) block_warps = 16;
-    return ieee_sqrt ? solve_occ<false>(p, block_warps, occupancy, async, grid_out, st)
-                     : solve_occ<true>(p, block_warps, occupancy, async, grid_out, st);
+    return ieee_sqrt ? solve_occ<false>(p, block_warps, occupancy, async, ctas_per_sm, grid_out, st)
+                     : solve_occ<true>(p, block_warps, occupancy, async, ctas_per_sm, grid_out, st);
 }
 
 

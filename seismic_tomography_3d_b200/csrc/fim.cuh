@@ -123,9 +123,25 @@ cudaError_t fim_init(float *T, size_t t_count, unsigned *qflag, size_t q_count, 
 cudaError_t fim_seed(const ShotDesc *shots, int nshots, const float *S, int gbx, int gbz, float *T,
                      unsigned *qflag, unsigned *lists, unsigned local_bits, unsigned *ctrl, cudaStream_t st,
                      size_t ring_cap = 0);
-// async: the asynchronous schedule (seeded with ring_cap = list_cap), else rounds.
+// async: the asynchronous schedule (seeded with ring_cap = list_cap), else rounds.  ctas_per_sm: of the
+// one-brick rounds kernel, 0: as many as fit.
 cudaError_t fim_solve(const FimLaunch &p, int block_warps, int occupancy, bool ieee_sqrt, int *grid_out,
-                      cudaStream_t st, bool async = false);
+                      cudaStream_t st, bool async = false, int ctas_per_sm = 0);
+// CTAs (of 16 warps) per SM of the one-brick rounds kernel; 0: as many as fit, two unless the caller
+// or the autotuner chose another shape (chosen), which is then taken as it is.  One for few bricks, since a round then lasts as long as its chain
+// of accesses and its barrier, which half the CTAs reach sooner.  A round's work is the bricks on
+// the shots' fronts (fronts: sum of n^(2/3) over shots of n bricks), and a large shot has fewer and
+// wider rounds than its share of them says.  ms per call, one CTA | two, by shots x bricks (fronts):
+//   1 x 67,626 (1,660) 0.713 | 0.791   2 x 67,626 (3,320)  0.986 | 1.020   3 x 67,626 (4,980)  1.280 | 1.278
+//   1 x 170,625 (3,077) 1.267 | 1.264  1 x 256,000 (4,032) 1.658 | 1.590   1 x 320,000 (4,680) 1.995 | 1.870
+//   10 x 8,788 (4,260) 0.629 | 0.645   13 x 8,788 (5,540)  0.702 | 0.701   15 x 8,788 (6,390)  0.734 | 0.727
+//   30 x 792 (2,570)   0.273 | 0.299   80 x 792 (6,850)    0.365 | 0.364   400 x 75 (7,110)    0.226 | 0.222
+constexpr unsigned long long kFewBricks = 170000;
+constexpr double kNarrowFronts = 5500.0;
+inline int rounds_ctas_per_sm(bool chosen, unsigned long long bricks, double fronts)
+{
+    return !chosen && bricks <= kFewBricks && fronts <= kNarrowFronts ? 1 : 0;
+}
 // One shot per thread-block cluster, its field in shared memory (k_fim_cluster): for a few shots
 // of at most *max_bricks bricks each (what the current device's shared memory holds).  Needs
 // neither seed nor pool reset; p.ctrl and p.stats zeroed.  bricks: of the largest shot.  An error means

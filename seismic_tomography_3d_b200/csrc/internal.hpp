@@ -37,6 +37,7 @@ struct EikPlan {
     int block_warps, occupancy;
     bool ieee_sqrt, async, brick8;
     long long cluster;  // bricks of the largest shot if each solves in a cluster, else 0
+    int ctas;           // CTAs per SM of the one-brick kernel, 0: as many as fit
     size_t t_total, q_total;
 };
 int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_window *windows, int nrec,
