@@ -507,7 +507,8 @@ def run_ours(args):
         SOLVER_RUN.update(schedule=3, block_warps=8, occupancy=3)
     elif not args.no_autotune:
         shape, tst = ctx.eik_autotune(sv.shots, windows=sv.windows, repeats=2)
-        tuned = dict(shape, trials=tst["trials"], best_ms=tst["best_ms"], default_ms=tst["default_ms"])
+        tuned = dict(shape, trials=tst["trials"], best_ms=tst["best_ms"], default_ms=tst["default_ms"],
+                     kept=tst["best_ms"] < tst["default_ms"])  # else the library's own choice runs
 
     def step_resident():
         _, st = ctx.eik_solve(sv.shots, windows=sv.windows, receivers=sv.receivers, want_recv=False, **SOLVER_RUN)
@@ -590,8 +591,7 @@ def run_ours(args):
     # DRAM bytes per brick activation from the committed ncu summary of the kernel that ran
     # (one capture of a 16-shot launch of the same workload), scaled to this launch's
     # activations
-    kernel = "k_fim_solve8" if stats[0]["nodes_per_brick"] == 512 else \
-        "k_fim_pair" if (tuned and tuned.get("schedule") == 3) or args.schedule == 3 else "k_fim_solve"
+    kernel = ctx.eik_kernel()
     per_act = DRAM_BYTES_PER_ACTIVATION.get(kernel)
     traffic = per_act * act if per_act else None
 

@@ -268,7 +268,7 @@ int tomo_eik_brick_shapes(int *xyz_triples, int cap);
 typedef struct {
     int trials;        /* launch shapes timed                                           */
     float best_ms;     /* device time of the persistent solve with the chosen shape      */
-    float default_ms;  /* the same with the built-in default shape                      */
+    float default_ms;  /* the same with the launch the library chooses by itself         */
 } tomo_tune_stats;
 
 /* Autotuner of the JW solve (no counterpart in the reference, whose launch shape is fixed).
@@ -280,8 +280,12 @@ typedef struct {
  * at the fastest 4x4x4 shape, the time band at 3, 6, 9 and 12 times the slowest brick
  * crossing (4 dx s_max; none is the shape's own time) and, if a band wins, the warps x
  * CTAs-per-SM shapes again with it.
- * Keeps the fastest in the context and writes it to *best (may be NULL).  Later solves on this context use the tuned value for every tomo_eik_opts field
- * they leave 0.  The traveltime pool holds the last trial's fields afterwards. */
+ * Writes the fastest to *best (may be NULL), times it once more in turn with the launch that the
+ * library chooses by itself, and keeps it in the context if it is faster: later solves on this
+ * context then use the tuned value for every tomo_eik_opts field they leave 0.  Otherwise the
+ * library goes on choosing (best_ms equals default_ms).  Batches that fit thread-block clusters
+ * (TOMO_SCHED_DEFAULT) keep them, unless a shape was faster than clusters on the batch tuned on.
+ * The traveltime pool holds the last trial's fields afterwards. */
 int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_window *windows,
                       int repeats, tomo_eik_opts *best, tomo_tune_stats *stats);
 

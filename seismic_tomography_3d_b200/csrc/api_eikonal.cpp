@@ -473,7 +473,8 @@ struct SolveCfg {
     float time_band;  // rounds schedule: time-band ordering (s), 0 = off
     unsigned long long spin_limit;  // polls of a device-side wait before it gives up
     bool brick8;      // 8^3 bricks (one CTA per 2 x 2 x 2 group of storage bricks)
-    bool plain;       // launch shape, schedule and wait limit all left to the library
+    bool asked;       // some of launch shape, schedule and wait limit is the caller's
+    bool plain;       // all of it is left to the library, and the autotuner chose none of it
     long long cluster;  // > 0: one cluster per shot, the largest of this many bricks (use_cluster)
     int ctas;           // one-brick rounds kernel: CTAs per SM, 0: as many as fit (choose_grid)
 };
@@ -516,9 +517,9 @@ SolveCfg solve_cfg(const tomo_ctx *ctx, const tomo_eik_opts *opts)
     const bool sched_default = !opts || opts->schedule == TOMO_SCHED_DEFAULT;
     c.pair = (opts && opts->schedule == TOMO_SCHED_PAIR) ||
              (sched_default && (ctx->tuned_schedule == TOMO_SCHED_PAIR || c.time_band > 0.f));
-    c.plain = sched_default && !(opts && (opts->block_warps > 0 || opts->occupancy > 0 || opts->brick > 0 ||
-                                          opts->spin_limit > 0)) &&
-              ctx->tuned_block_warps == 0 && ctx->tuned_schedule == 0 && ctx->tuned_brick == 0;
+    c.asked = !sched_default || (opts && (opts->block_warps > 0 || opts->occupancy > 0 || opts->brick > 0 ||
+                                          opts->spin_limit > 0));
+    c.plain = !c.asked && ctx->tuned_block_warps == 0 && ctx->tuned_schedule == 0 && ctx->tuned_brick == 0;
     c.spin_limit = (opts && opts->spin_limit > 0) ? opts->spin_limit : kSpinLimit;
     // Brick shape: 4^3 unless asked for (or tuned to) 8^3.  The 8^3 kernel runs the rounds
     // schedule without the time band.
@@ -612,18 +613,25 @@ int make_batch(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_wi
     return TOMO_OK;
 }
 
-// Whether a batch solves with one cluster per shot (k_fim_cluster): the bricks of its largest
-// shot, or 0.  For shots that fit a cluster's shared memory, no more of them than the GPU runs at
-// once, no time band, and nothing of the launch asked for by the caller or the autotuner.  Four
+// The bricks of a batch's largest shot if each shot could solve in a cluster (k_fim_cluster), or 0:
+// for shots that fit a cluster's shared memory, no more of them than the GPU runs at once.  Four
 // clusters run side by side; with eight shots of 360, 3,375 and 8,788 bricks the call takes 0.192 |
 // 0.193, 0.380 | 0.373 and 0.699 | 0.588 ms against one grid.
-long long use_cluster(const tomo_ctx *ctx, const Batch &bt, const SolveCfg &c)
+long long fits_clusters(const tomo_ctx *ctx, const Batch &bt)
 {
     constexpr size_t kMaxShots = 4;
-    if (!c.plain || c.time_band > 0.f || bt.sd.size() > kMaxShots) return 0;
+    if (bt.sd.size() > kMaxShots) return 0;
     long long most = 0;
     for (const ShotDesc &d : bt.sd) most = std::max(most, (long long)d.nbx * d.nby * d.nbz);
     return most <= ctx->cluster_bricks ? most : 0;
+}
+
+// Whether it does: no time band, nothing of the launch asked for by the caller, and no shape that
+// the autotuner found faster than clusters on a batch that fits them.
+void use_cluster(const tomo_ctx *ctx, const Batch &bt, SolveCfg &c)
+{
+    c.cluster = c.asked || c.time_band > 0.f || ctx->tuned_beats_cluster ? 0 : fits_clusters(ctx, bt);
+    if (c.cluster) c.brick8 = c.pair = false;  // a shape tuned on a batch that does not fit
 }
 
 // Unbanded batches of many bricks run two bricks per warp at 8 warps x 3 CTAs per SM, when nothing
@@ -842,7 +850,7 @@ int eik_plan(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tomo_wind
     Batch bt;
     int rc = make_batch(ctx, nshots, shots, windows, nrec, receivers, bt);
     if (rc != TOMO_OK) return rc;
-    cfg.cluster = use_cluster(ctx, bt, cfg);
+    use_cluster(ctx, bt, cfg);
     choose_pair(bt, cfg);
     choose_grid(bt, cfg);
     rc = upload_batch(ctx, bt, nrec, receivers);
@@ -904,7 +912,7 @@ int tomo_eik_solve(tomo_ctx *ctx, int nshots, const tomo_point *shots, const tom
     Batch bt;
     int rc = make_batch(ctx, nshots, shots, windows, nrec, receivers, bt);
     if (rc != TOMO_OK) return rc;
-    cfg.cluster = use_cluster(ctx, bt, cfg);
+    use_cluster(ctx, bt, cfg);
     choose_pair(bt, cfg);
     choose_grid(bt, cfg);
     ctx->have_solve = false;  // the pool is about to be overwritten
@@ -1084,6 +1092,7 @@ int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const 
     ctx->tuned_brick = 0;
     ctx->tuned_schedule = 0;
     ctx->tuned_time_band = 0.f;
+    ctx->tuned_beats_cluster = false;
     const int warps[] = {kDefaultBlockWarps, 8, 4};
     const int occs[] = {4, 5, 6, 3};
     const int inners[] = {16, 8, 32};
@@ -1091,10 +1100,13 @@ int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const 
     o.op = TOMO_OP_JW;
     o.brick = TOMO_BRICK_4;
     tomo_eik_stats st{};
-    // warm-up (first launch of each kernel variant pays for module loading)
-    int rc = tomo_eik_solve(ctx, nshots, shots, windows, 0, nullptr, nullptr, &o, &st);
+    // warm-up (first launch of each kernel variant pays for module loading): the launch the library
+    // chooses when nothing is asked for or tuned, which the chosen shape is up against below
+    const tomo_eik_opts untuned{};
+    int rc = tomo_eik_solve(ctx, nshots, shots, windows, 0, nullptr, nullptr, &untuned, &st);
     if (rc != TOMO_OK) return rc;
-    float best_ms = 0.f, default_ms = 0.f;
+    const bool clusters = ctx->eik_kernel == TOMO_KERNEL_CLUSTER;
+    float best_ms = 0.f;
     int trials = 0, bw = kDefaultBlockWarps, bo = kDefaultOccupancy, bi = kDefaultMaxInner;
     for (int w : warps)
         for (int oc : occs)
@@ -1109,7 +1121,6 @@ int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const 
                     if (r == 0) continue;  // first launch of this variant: not timed
                     ms = (r == 1) ? st.solve_ms : std::min(ms, st.solve_ms);
                 }
-                if (trials == 0) default_ms = ms;
                 if (trials == 0 || ms < best_ms) {
                     best_ms = ms;
                     bw = w;
@@ -1246,26 +1257,45 @@ int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const 
         bw = pw;
         bo = po;
     }
-    ctx->tuned_brick = bbrick;
-    ctx->tuned_schedule = pair_best ? TOMO_SCHED_PAIR : 0;
-    ctx->tuned_block_warps = bw;
-    ctx->tuned_occupancy = bo;
-    ctx->tuned_max_inner = bi;
-    ctx->tuned_time_band = bb;
-    if (best) {
-        *best = tomo_eik_opts{};
-        best->op = TOMO_OP_JW;
-        best->brick = bbrick;
-        best->block_warps = bw;
-        best->occupancy = bo;
-        best->max_inner = bi;
-        best->time_band = bb;
-        best->schedule = pair_best ? TOMO_SCHED_PAIR : TOMO_SCHED_DEFAULT;
+    tomo_eik_opts tuned{};
+    tuned.op = TOMO_OP_JW;
+    tuned.brick = bbrick;
+    tuned.block_warps = bw;
+    tuned.occupancy = bo;
+    tuned.max_inner = bi;
+    tuned.time_band = bb;
+    tuned.schedule = pair_best ? TOMO_SCHED_PAIR : TOMO_SCHED_DEFAULT;
+    if (best) *best = tuned;
+    // The chosen shape against the untuned launch, in turn, with the set-up (clusters need no pool
+    // reset), and kept only if it is faster: the best of 50 shapes is a lucky one, and the untuned
+    // launch may be one that no shape above is (clusters, two bricks per warp, one CTA per SM).
+    float untuned_ms = 0.f, untuned_call = 0.f, chosen_ms = 0.f, chosen_call = 0.f;
+    for (int r = 0; r < std::max(repeats, 3) + 1; r++) {
+        tomo_eik_stats su{}, sc{};
+        rc = tomo_eik_solve(ctx, nshots, shots, windows, 0, nullptr, nullptr, &untuned, &su);
+        if (rc == TOMO_OK) rc = tomo_eik_solve(ctx, nshots, shots, windows, 0, nullptr, nullptr, &tuned, &sc);
+        if (rc != TOMO_OK) return rc;
+        if (r == 0) continue;
+        auto least = [r](float &best_so_far, float ms) { best_so_far = r == 1 ? ms : std::min(best_so_far, ms); };
+        least(untuned_ms, su.solve_ms);
+        least(untuned_call, su.setup_ms + su.solve_ms);
+        least(chosen_ms, sc.solve_ms);
+        least(chosen_call, sc.setup_ms + sc.solve_ms);
+    }
+    const bool keep = chosen_call < untuned_call;
+    if (keep) {
+        ctx->tuned_brick = bbrick;
+        ctx->tuned_schedule = pair_best ? TOMO_SCHED_PAIR : 0;
+        ctx->tuned_block_warps = bw;
+        ctx->tuned_occupancy = bo;
+        ctx->tuned_max_inner = bi;
+        ctx->tuned_time_band = bb;
+        ctx->tuned_beats_cluster = clusters;
     }
     if (stats) {
         stats->trials = trials;
-        stats->best_ms = best_ms;
-        stats->default_ms = default_ms;
+        stats->best_ms = keep ? std::min(chosen_ms, untuned_ms) : untuned_ms;
+        stats->default_ms = untuned_ms;
     }
     return TOMO_OK;
 }

@@ -98,6 +98,7 @@ struct tomo_ctx {
     bool have_solve = false;
     // launch shape chosen by tomo_eik_autotune (0: not tuned)
     int cluster_bricks = 0;       // largest shot one cluster can hold (fim_cluster_limit)
+    bool tuned_beats_cluster = false;  // the tuned shape was faster than clusters on a batch that fits them
     int eik_kernel = 0;           // TOMO_KERNEL_* of the last solve
     int tuned_block_warps = 0, tuned_occupancy = 0, tuned_max_inner = 0;
     int tuned_brick = 0;          // 0: none chosen (4^3); TOMO_BRICK_4 / TOMO_BRICK_8

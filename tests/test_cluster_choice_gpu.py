@@ -80,3 +80,30 @@ def test_iteration_reports_its_solve(tomo):
             assert ctx.eik_kernel() == "k_fsm"
             ctx.iteration(sv.shots, sv.receivers, (2 * sv.h,) * 3, cg_iterations=3)
             assert ctx.eik_kernel() == "k_fim_cluster"
+
+
+def test_autotuned_context_keeps_clusters(tomo):
+    """A shape tuned on a batch that clusters solve faster is not kept; one tuned on a larger
+    batch leaves the small batches their clusters; what the caller asks for is always taken."""
+    small, n = wl.small(3, 33, 29, 17), (33, 29, 17)
+    with tomo.Context(*n, small.h) as ctx:
+        ctx.set_velocity(small.velocity)
+        _, st = ctx.eik_autotune(small.shots)
+        assert 0 < st["best_ms"] <= st["default_ms"]
+        ctx.eik_solve(small.shots)
+        assert ctx.eik_kernel() == "k_fim_cluster"
+    many = wl.small(3, 60, 60, 40, nshots=24)
+    with tomo.Context(60, 60, 40, many.h) as ctx:
+        ctx.set_velocity(many.velocity)
+        shape, st = ctx.eik_autotune(many.shots)
+        assert 0 < st["best_ms"] <= st["default_ms"]
+        banded = st["best_ms"] < st["default_ms"] and shape["time_band"] > 0
+        ctx.eik_solve(many.shots[:2])
+        # a tuned time band applies to every later solve, and clusters run without one
+        assert ctx.eik_kernel() == ("k_fim_pair" if banded else "k_fim_cluster")
+        T = ctx.eik_volume(1)
+        ctx.eik_solve(many.shots[:2], schedule=1, brick=1)
+        assert ctx.eik_kernel() == "k_fim_solve"
+        np.testing.assert_allclose(ctx.eik_volume(1), T, rtol=1e-5, atol=1e-6)
+        ctx.eik_solve(many.shots)
+        assert ctx.eik_kernel() != "k_fim_cluster"
