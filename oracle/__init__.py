@@ -228,8 +228,14 @@ def have_ref(gpu=False):
     return os.path.exists(os.path.join(_REF, "libref_fim.so" if gpu else "libref_eik.so"))
 
 
+class ReferenceNotBuilt(OSError):
+    """Neither the reference's solvers (oracle/_ref) nor the sources to build them are here."""
+
+
 def _load_ref(gpu=False):
     global _ref_eik, _ref_fim
+    if not have_ref(gpu) and not reference_src():
+        raise ReferenceNotBuilt("oracle/_ref (the reference's own solvers) not built, and its sources are not here")
     if gpu:
         if _ref_fim is None:
             _ref_fim = ctypes.CDLL(os.path.join(_REF, "libref_fim.so"))
