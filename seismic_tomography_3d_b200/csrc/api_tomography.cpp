@@ -74,6 +74,16 @@ std::vector<float> gaussian_weights(int samples, float stdv)
     return k;
 }
 
+// Filter size that model_update takes on by itself: 1 for none, 0 where gaussian_smooth is needed.
+// A single sample leaves dm as it is unless its weight, 1 / sum of itself, is NaN (a standard
+// deviation whose square leaves the FP32 range).
+int fused_samples(int smooth, int samples, float stdv)
+{
+    if (!smooth) return 1;
+    if (samples == 1 && gaussian_weights(1, stdv)[0] != 1.0f) return 0;
+    return tomo::update_fuses(samples) ? samples : 0;
+}
+
 int bits_for(long long n)
 {
     int b = 1;
@@ -629,7 +639,7 @@ int update_prepare(tomo_ctx *ctx, const tomo_update_opts *opts)
         CK(ctx->gauss_kernel.ensure(k.size()));
         CK(cudaMemcpyAsync(ctx->gauss_kernel.ptr, k.data(), k.size() * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-        if (!tomo::update_fuses(samples)) CK(ctx->dm_smooth.ensure(n));
+        if (!fused_samples(smooth, samples, stdv)) CK(ctx->dm_smooth.ensure(n));
         CK(cudaStreamSynchronize(ctx->stream));  // k is a host temporary
     }
     return TOMO_OK;
@@ -647,8 +657,8 @@ int update_enqueue_v(tomo_ctx *ctx, const tomo_update_opts *opts, float *velocit
     CK(tomo::model_dm(ctx->x.ptr, ctx->dm.ptr, g.nx, g.ny, g.nz, g.dx, g.dy, g.dz, ctx->dxt, ctx->dyt, ctx->dzt,
                       ctx->nxt, ctx->nyt, ctx->nzt, m, ctx->stream));
     const float *dm = ctx->dm.ptr;
-    int fused = smooth ? samples : 1;
-    if (!tomo::update_fuses(fused)) {
+    int fused = fused_samples(smooth, samples, opts ? opts->standard_deviation : 2.0f);
+    if (!fused) {
         CK(tomo::gaussian_smooth(ctx->dm.ptr, ctx->dm_smooth.ptr, g.nx, g.ny, g.nz, samples, ctx->gauss_kernel.ptr,
                                  ctx->stream));
         dm = ctx->dm_smooth.ptr;
