@@ -88,7 +88,8 @@ typedef struct {
     int sweep_groups;/* TOMO_OP_NGB schedule.  0 (default): tile wavefront -- one warp
                         (eight where the tiles in flight are few, as for one shot) per
                         16x8x8 tile of a sweep in shared memory, tiles in diagonal
-                        order behind their upwind tiles, one grid barrier per sweep;
+                        order behind their upwind tiles, a shot's sweeps ordered by
+                        its count of finished tiles (eight warps: a grid barrier);
                         batches with a source on the last node of its window along an
                         axis take the plane schedule.  > 0: the diagonal-plane schedule
                         (a barrier per plane) with that many independent block groups

@@ -1216,7 +1216,7 @@ int tomo_eik_autotune(tomo_ctx *ctx, int nshots, const tomo_point *shots, const 
             if (ms < best_ms) {
                 best_ms = ms;
                 bb = o.time_band;
-                pair_best = false;  // a banded solve runs the one-brick kernel
+                pair_best = false;  // a banded solve runs two bricks per warp by itself
             }
             ++trials;
         }

@@ -30,7 +30,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kLongRow = 256;  // A' rows with more non-zeros are summed by a whole block
+constexpr int kLongRow = 256;  // A' rows of no more non-zeros are never long ones (long_row_limit)
 
 // Block-wide FP64 sum in a fixed order; result valid in every thread.
 __device__ __forceinline__ double block_sum(double v, double *sh)
@@ -60,7 +60,8 @@ __device__ __forceinline__ double grid_sum(const double *partials, int nb, doubl
     return v;
 }
 
-// Rows of A' longer than this are summed by whole blocks (t_ptr[M] = the non-zero count).
+// Rows of A' longer than this are long ones, summed with eight accumulators a lane (spmv_t;
+// t_ptr[M] = the non-zero count).
 __device__ __forceinline__ int long_row_limit(const int *t_ptr, int M)
 {
     const long long mean8 = 8ll * t_ptr[M] / (M > 0 ? M : 1);

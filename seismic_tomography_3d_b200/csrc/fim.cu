@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(512) __maxnreg__(fim_regs(MINB)) k_fim_solve(F
 
 // ---------------------------------------------------------------------------------------
 // Small batches: one shot per thread-block cluster, its whole field in the cluster's shared
-// memory (FimLaunch of a batch whose shots each fit, fim_cluster_fits).
+// memory (batches whose shots each fit: fits_clusters in api_eikonal.cpp).
 //
 // A shot of a few thousand bricks has tens to hundreds of them to relax in a round, so a round
 // of k_fim_solve lasts as long as its chain of dependent accesses to L2 -- list count, item,
@@ -766,7 +766,8 @@ __global__ void __launch_bounds__(512) __maxnreg__(fim_regs(MINB)) k_fim_solve(F
 // shared memory; queueing a brick sets its owner's bit, a reduction nobody waits for (flags,
 // counts and lists as in k_fim_solve cost two round trips more at the end of an item); a round
 // ends at the hardware's cluster barrier, every warp finds the CTA's bricks of the round in the
-// 24 words of its bit map, and the field is written to the pool once, at the end.  Rounds, in-brick relaxation,
+// 32 words of its bit map (one per lane: kClusterMaxCap bricks, of which shared memory holds 798),
+// and the field is written to the pool once, at the end.  Slowness stays in global memory.  Rounds, in-brick relaxation,
 // queueing tests and tolerances are those of k_fim_solve.  Clusters do not wait for each other
 // (no cooperative launch).  ms per call, against one grid of 148 CTAs: 360 bricks 0.134 | 0.175 (1 to
 // 4 shots alike), 1,000 0.176 | 0.258, 3,375 0.232 | 0.298, 8,788 0.370 | 0.391.

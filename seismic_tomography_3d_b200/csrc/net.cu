@@ -537,7 +537,7 @@ __device__ __forceinline__ void axis_weight(int x, int k, int n, int &c0, int &c
 // where x enters a new cell.  Lanes follow z, the fastest axis, across column ends, so no
 // lane idles on a depth that is not a multiple of 32.  64 windows of 201 x 201 x 101 at
 // stride 4 (261 M nodes): the kernel 3.70 -> 0.52 ms (0.71 with IEEE root and
-// division and runs of 32), 83 % of the issue slots.
+// division and runs of 32); issue in 76 % of the slots on 8 windows.
 constexpr int kTimeRun = 64;
 
 // kFast: the short root of common.cuh and 32-bit (z, y) pairs; else the IEEE root and 64 bits (a

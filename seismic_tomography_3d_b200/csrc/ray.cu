@@ -89,10 +89,11 @@ struct Field {
 // kPrepared: divisions by prepared divisors (common.cuh) instead of IEEE divisions, the same
 // quotients in 3 instructions of 12.  A step has twelve: nine by the grid and cell spacings,
 // prepared once per thread, and three by the gradient's norm, which share one reciprocal.  The
-// march is bound by issue (316 instructions a step), and its divisions were a third of them:
+// march is bound by issue, and its divisions were a third of its instructions (346 thread
+// instructions a step before, 229 now, issuing in 61 % of the slots):
 // 160,000 rays of the 201 x 201 x 101 model 2.2 -> 1.5 ms, of the 401 x 401 x 201 model 4.4 ->
-// 3.4 ms, the second 3.0 ms with 4 CTAs an SM, whose rays share more of L1 (7 fit; 6: 3.1, 5:
-// 3.1, 8 with spills: 4.2).  Only quotients of time differences under 2^-80 s would not be exact; such a
+// 3.4 ms, the second 3.0 ms with registers for at least 4 CTAs an SM (5 fit then, whose rays share
+// more of L1; for at least 5: 3.1, 6: 3.1, 8 with spills: 4.2).  Only quotients of time differences under 2^-80 s would not be exact; such a
 // component moves no position by an ulp.  Chosen when all spacings lie in [kDivMin, kDivMax]
 // (metres); outside it a reciprocal or a remainder could leave the FP32 range.
 template <class I, bool kPrepared>
